@@ -387,6 +387,18 @@ __device__ __forceinline__ Phys<R> make_phys(const PhysArgs& pa)
   return ph;
 }
 
+// What all threads of a leaf share, in the bytes behind the tile barrier
+template <typename R>
+struct LeafScalars {
+  R dt, dtdx, dtdy;
+  int visc;
+};
+template <typename R>
+__device__ __forceinline__ LeafScalars<R>& leaf_scalars()
+{
+  return *reinterpret_cast<LeafScalars<R>*>(w2d_smem + 64);
+}
+
 // Pulls block b of pool src (NEQ*400 values) into shared tile dst; every
 // thread returns whether the copy completed (false: timeout recorded).
 template <typename R, int NEQ>
@@ -433,9 +445,7 @@ __device__ __forceinline__ bool wait_tiles(uint64_t* bar, int* err, int b)
 // then spill a few registers (about 60 and 110 bytes of spill loads) but
 // keep 4 CTAs (36 warps) per SM instead of 3, which measured 12% (half) and
 // 7% (full) faster: the FP64 pipe waits less on the long division and
-// square-root chains.  (The FP64 full step gathers its fill II ghosts after
-// its tiles have landed rather than during the copy: fewer values live
-// across the wait, half the spills, 1.7% faster.)  In FP32, 5 and 6 CTAs
+// square-root chains.  In FP32, 5 and 6 CTAs
 // per SM (40 and 32 registers, 150-210 bytes of spill loads in the full
 // step) measured 3% and 13% slower on the 256-run ensemble than 4.
 template <typename R>
@@ -500,6 +510,29 @@ __device__ __forceinline__ double d_cooldmc(const double* __restrict__ tab, doub
   return (c1 - c0) * (T - T0) / (T1 - T0) + c0;
 }
 
+// Warp maximum of values >= 0 through the integer order of their bit patterns
+// (redux.sync: one instruction for a float, two and a select for a double,
+// against five shuffle rounds).  As fmax does, a NaN gives way to any number;
+// a warp of NaNs gives 0, or NaN with KEEP_NAN.
+template <bool KEEP_NAN = false>
+__device__ __forceinline__ double warp_max0(double x)
+{
+  const bool num = x >= 0.;
+  const unsigned hi = num ? (unsigned)__double2hiint(x) : 0u, lo = num ? (unsigned)__double2loint(x) : 0u;
+  const unsigned mh = __reduce_max_sync(0xffffffffu, hi);
+  const unsigned ml = __reduce_max_sync(0xffffffffu, hi == mh ? lo : 0u);
+  if (KEEP_NAN && !__any_sync(0xffffffffu, num)) return x;
+  return __hiloint2double((int)mh, (int)ml);
+}
+template <bool KEEP_NAN = false>
+__device__ __forceinline__ float warp_max0(float x)
+{
+  const bool num = x >= 0.f;
+  const unsigned m = __reduce_max_sync(0xffffffffu, num ? __float_as_uint(x) : 0u);
+  if (KEEP_NAN && !__any_sync(0xffffffffu, num)) return x;
+  return __uint_as_float(m);
+}
+
 // Per-block statistics of a primitive tile (cells 0..17 valid): the CFL
 // partial of timestep (src/timestep.f90:21-47), the criteria maximum
 // (src/criteria.f90:16-50) and, under DMC, the cooling-time limit.  Both
@@ -513,14 +546,15 @@ __device__ __forceinline__ void block_stats(const R (*sp)[W2D_W][W2D_W], const P
                                             const PhysArgs& pa, int b, double* sred)
 {
   const int tid = threadIdx.x;
-  double au = 0., av = 0., grad = 0., dtc = 1e30;
+  R au = R(0.), av = R(0.), grad = R(0.);
+  double dtc = 1e30;
   if (tid < 256) {
     const int i = 1 + tid % 16, j = 1 + tid / 16;
     const int ti = i + 1, tj = j + 1;
     const R rho = sp[0][tj][ti], vx = sp[1][tj][ti], vy = sp[2][tj][ti], p = sp[3][tj][ti];
     const R cs = sound(ph, p, rho);
-    au = (double)(absr(vx) + cs);
-    av = (double)(absr(vy) + cs);
+    au = absr(vx) + cs;
+    av = absr(vy) + cs;
     const R fl = R(1e-15);
     const R am = fmaxr(fl, absr(p)), am2 = fmaxr(fl, absr(rho));
     R dp = absr(sp[3][tj][ti + 1] - p);
@@ -531,7 +565,7 @@ __device__ __forceinline__ void block_stats(const R (*sp)[W2D_W][W2D_W], const P
     dr = fmaxr(dr, absr(sp[0][tj][ti - 1] - rho));
     dr = fmaxr(dr, absr(sp[0][tj + 1][ti] - rho));
     dr = fmaxr(dr, absr(sp[0][tj - 1][ti] - rho));
-    grad = (double)fmaxr(divr(dp, am), divr(dr, am2));
+    grad = fmaxr(divr(dp, am), divr(dr, am2));
     if (pa.cooling == COOL_DMC) {                    // src/timestep.f90:34-41
       const double T = ((double)p / (double)rho) * pa.tempsc;
       if (T > 1e4) {
@@ -540,17 +574,17 @@ __device__ __forceinline__ void block_stats(const R (*sp)[W2D_W][W2D_W], const P
       }
     }
   }
+  au = warp_max0(au);
+  av = warp_max0(av);
+  grad = warp_max0(grad);
+  if (pa.cooling == COOL_DMC) {
 #pragma unroll
-  for (int o = 16; o > 0; o >>= 1) {
-    au = fmax(au, __shfl_xor_sync(0xffffffffu, au, o));
-    av = fmax(av, __shfl_xor_sync(0xffffffffu, av, o));
-    grad = fmax(grad, __shfl_xor_sync(0xffffffffu, grad, o));
-    dtc = fmin(dtc, __shfl_xor_sync(0xffffffffu, dtc, o));
+    for (int o = 16; o > 0; o >>= 1) dtc = fmin(dtc, __shfl_xor_sync(0xffffffffu, dtc, o));
   }
   if ((tid & 31) == 0) {
-    sred[tid >> 5] = au;
-    sred[16 + (tid >> 5)] = av;
-    sred[32 + (tid >> 5)] = grad;
+    sred[tid >> 5] = (double)au;
+    sred[16 + (tid >> 5)] = (double)av;
+    sred[32 + (tid >> 5)] = (double)grad;
     sred[48 + (tid >> 5)] = dtc;
   }
   __syncthreads();
@@ -578,24 +612,26 @@ __device__ __forceinline__ void block_stats(const R (*sp)[W2D_W][W2D_W], const P
 // covers the neighbour pairs inside the interior here; fill I folds in the
 // pairs of edge cells with their layer-0 ghosts (fill_face_stats).  The
 // two parts combine exactly: for am > 0, max(RN(x/am), RN(y/am)) =
-// RN(max(x, y)/am).  st (its interior) and sred are overwritten.
+// RN(max(x, y)/am).  st (its interior) is overwritten.
+//
+// The warps' maxima go to sred; stats_finish combines them after the next CTA
+// barrier (the one that ends the leaf), in the warp that has no cells here,
+// while the others go on to the next leaf.
 template <typename R, int NEQ>
-__device__ __forceinline__ void interior_stats(R (*st)[W2D_W][W2D_W], double* sred, const Phys<R>& ph,
-                                               const KArgs& a, int b, int lev)
+__device__ __forceinline__ void interior_stats(R (*st)[W2D_W][W2D_W], double* sred, const Phys<R>& ph)
 {
   const int tid = threadIdx.x;
   const int i = 1 + tid % 16, j = 1 + tid / 16;
   const int ti = i + 1, tj = j + 1;
-  double au = 0., av = 0., grad = 0.;
-  R rho = R(0.), p = R(0.);
+  R au = R(0.), av = R(0.), rho = R(0.), p = R(0.);
   if (tid < 256) {
     R q[NEQ], nv[NEQ], T;
 #pragma unroll
     for (int k = 0; k < NEQ; ++k) nv[k] = st[k][tj][ti];
     uprim<NEQ>(ph, q, nv, T);
     const R cs = sound(ph, q[3], q[0]);
-    au = (double)(absr(q[1]) + cs);
-    av = (double)(absr(q[2]) + cs);
+    au = absr(q[1]) + cs;
+    av = absr(q[2]) + cs;
     rho = q[0];
     p = q[3];
     // (this cell's entries of st are read by no other thread before the
@@ -612,27 +648,33 @@ __device__ __forceinline__ void interior_stats(R (*st)[W2D_W][W2D_W], double* sr
     if (i > 1) { dp = fmaxr(dp, absr(st[3][tj][ti - 1] - p)); dr = fmaxr(dr, absr(st[0][tj][ti - 1] - rho)); }
     if (j < W2D_NX) { dp = fmaxr(dp, absr(st[3][tj + 1][ti] - p)); dr = fmaxr(dr, absr(st[0][tj + 1][ti] - rho)); }
     if (j > 1) { dp = fmaxr(dp, absr(st[3][tj - 1][ti] - p)); dr = fmaxr(dr, absr(st[0][tj - 1][ti] - rho)); }
-    grad = (double)fmaxr(divr(dp, am), divr(dr, am2));
-  }
-#pragma unroll
-  for (int o = 16; o > 0; o >>= 1) {
-    au = fmax(au, __shfl_xor_sync(0xffffffffu, au, o));
-    av = fmax(av, __shfl_xor_sync(0xffffffffu, av, o));
-    grad = fmax(grad, __shfl_xor_sync(0xffffffffu, grad, o));
-  }
-  if ((tid & 31) == 0) {
-    sred[tid >> 5] = au;
-    sred[16 + (tid >> 5)] = av;
-    sred[32 + (tid >> 5)] = grad;
-  }
-  __syncthreads();
-  if (tid == 0) {
-    double m0 = sred[0], m1 = sred[16], m2 = sred[32];
-    for (int w = 1; w < W2D_THREADS / 32; ++w) {
-      m0 = fmax(m0, sred[w]);
-      m1 = fmax(m1, sred[16 + w]);
-      m2 = fmax(m2, sred[32 + w]);
+    const R grad = warp_max0(fmaxr(divr(dp, am), divr(dr, am2)));
+    au = warp_max0(au);
+    av = warp_max0(av);
+    if ((tid & 31) == 0) {
+      sred[tid >> 5] = (double)au;
+      sred[8 + (tid >> 5)] = (double)av;
+      sred[16 + (tid >> 5)] = (double)grad;
     }
+  }
+}
+
+template <typename R>
+__device__ __forceinline__ void stats_finish(const double* sred, const KArgs& a, int b)
+{
+  const int lane = (int)threadIdx.x - 256;
+  if (lane < 0) return;
+  double m0 = 0., m1 = 0., m2 = 0.;
+  if (lane < 8) {
+    m0 = sred[lane];
+    m1 = sred[8 + lane];
+    m2 = sred[16 + lane];
+  }
+  m0 = warp_max0(m0);
+  m1 = warp_max0(m1);
+  m2 = warp_max0(m2);
+  if (lane == 0) {
+    const int lev = a.lev[b];
     const R t1 = R(geo_dx(a, b, lev)) / R(m0);
     const R t2 = R(geo_dy(a, b, lev)) / R(m1);
     a.cfl[b] = (double)fminr(t1, t2);
@@ -696,16 +738,25 @@ __device__ __forceinline__ bool half_leaf(const KArgs& a, const PhysArgs& pa, do
   const R* __restrict__ u = (const R*)a.u + (size_t)b * bs;
   R* __restrict__ up = (R*)a.up + (size_t)b * bs;
   if (tid == 0) tile_issue<R, NEQ>(&su[0][0][0], dmc ? (const R*)a.prim + (size_t)b * bs : u, bar);
-  const int lev = a.lev[b];
-  const double dtm = step_dt(a, b, dt) / 2.;
-  const R dtdx = R(dtm / geo_dx(a, b, lev));
-  const R dtdy = R(dtm / geo_dy(a, b, lev));
+  // dt/2, dt/(2 dx) and dt/(2 dy) of the block, once for all its threads
+  // (read after the barriers below)
+  LeafScalars<R>& sc = leaf_scalars<R>();
+  if (tid == W2D_THREADS - 1) {
+    const int lev = a.lev[b];
+    const double dtm = step_dt(a, b, dt) / 2.;
+    sc.dt = R(dtm);
+    sc.dtdx = R(dtm / geo_dx(a, b, lev));
+    sc.dtdy = R(dtm / geo_dy(a, b, lev));
+  }
   if (!wait_tiles_p<U>(bar, a.err, b, par)) return false;
 
-  // primitives (in place) and sound speed of cells 0..17 (corners skipped)
-  for (int c = tid; c < 18 * 18; c += W2D_THREADS) {
-    const int ti = 1 + c % 18, tj = 1 + c / 18;
-    if ((ti == 1 || ti == 18) && (tj == 1 || tj == 18)) continue;
+  // primitives and sound speed of cells 0..17 (corners skipped): the first
+  // eight warps take the interior, the ninth the 64 edge ghosts
+  for (int c = tid; c < 320; c += tid < 256 ? 320 : 32) {
+    int ti = 1 + c % 16, tj = 1 + c / 16;
+    if (c >= 256) ghost_ij((c - 256) / 16, 0, 1 + c % 16, ti, tj);
+    ++ti;
+    ++tj;
     R q[NEQ];
 #pragma unroll
     for (int k = 0; k < NEQ; ++k) q[k] = su[k][tj][ti];
@@ -747,14 +798,15 @@ __device__ __forceinline__ bool half_leaf(const KArgs& a, const PhysArgs& pa, do
 
   if (tid < 256) {  // src/step.f90:20-40
     const int i = 1 + tid % 16, j = 1 + tid / 16;
+    const R dtdx = sc.dtdx, dtdy = sc.dtdy;
     R S[NEQ];
-    if (pa.cyl) cyl_sources<R, NEQ>(st, i + 1, j + 1, R(cyl_radius(a, b, lev, j)), ph.cv, S);
+    if (pa.cyl) cyl_sources<R, NEQ>(st, i + 1, j + 1, R(cyl_radius(a, b, a.lev[b], j)), ph.cv, S);
 #pragma unroll
     for (int k = 0; k < NEQ; ++k) {
       // u from the tile (under DMC the tile holds the primitives: u from HBM)
       const R uo = dmc ? u[k * W2D_CELLS + cidx(i, j)] : su[k][j + 1][i + 1];
       R v = uo - dtdx * (sf[k][j - 1][i] - sf[k][j - 1][i - 1]) - dtdy * (sg[k][j][i - 1] - sg[k][j - 1][i - 1]);
-      if (pa.cyl) v = v + R(dtm) * S[k];
+      if (pa.cyl) v = v + sc.dt * S[k];
       up[k * W2D_CELLS + cidx(i, j)] = v;
     }
   }
@@ -779,7 +831,7 @@ __global__ void __launch_bounds__(W2D_THREADS, w2d_minb<R>(P)) k_half(KArgs a, P
 template <typename R, int NEQ>
 __host__ __device__ constexpr size_t smem_full()
 {
-  return 128 + sizeof(R) * (2 * NEQ * W2D_CELLS + 2 * NEQ * 272);
+  return 128 + 192 + sizeof(R) * (2 * NEQ * W2D_CELLS + 2 * NEQ * 272);
 }
 
 // One leaf of the full step (position li of the leaf list).  Returns false
@@ -792,6 +844,7 @@ __device__ __forceinline__ bool full_leaf(const KArgs& a, const PhysArgs& pa, do
   R(*so)[W2D_W][W2D_W] = reinterpret_cast<R(*)[W2D_W][W2D_W]>(w2d_smem + 128 + sizeof(R) * NEQ * W2D_CELLS);
   R(*sf)[16][17] = reinterpret_cast<R(*)[16][17]>(w2d_smem + 128 + sizeof(R) * 2 * NEQ * W2D_CELLS);
   R(*sg)[17][16] = reinterpret_cast<R(*)[17][16]>(w2d_smem + 128 + sizeof(R) * (2 * NEQ * W2D_CELLS + NEQ * 272));
+  double* sred = reinterpret_cast<double*>(w2d_smem + 128 + sizeof(R) * (2 * NEQ * W2D_CELLS + 2 * NEQ * 272));
   const Phys<R> ph = make_phys<R, SOLVER, LIMITER>(pa);
   const int tid = threadIdx.x;
   const size_t bs = (size_t)NEQ * W2D_CELLS;
@@ -799,68 +852,63 @@ __device__ __forceinline__ bool full_leaf(const KArgs& a, const PhysArgs& pa, do
   const int b = a.leaves[li];
   R* __restrict__ u = (R*)a.u + (size_t)b * bs;
   if (tid == 0) tiles_issue2<R, NEQ>(&st[0][0][0], upool + (size_t)b * bs, &so[0][0][0], u, bar);
-  const int lev = a.lev[b];
-  const double dtb = step_dt(a, b, dt);
-  const R dtdx = R(dtb / geo_dx(a, b, lev));
-  const R dtdy = R(dtb / geo_dy(a, b, lev));
-  const bool visc = lev >= (geo_nlevs(a, b) - 1);
-  const R eta = R(a.eta);
-
-  // ghosts of the filled up gathered from the pool (box faces read the
-  // block's own interior there too): in FP32 while the tiles land; in FP64
-  // after them, with fewer values live across the wait (there the step's
-  // register pressure costs more than the copy's latency)
-  constexpr bool early = sizeof(R) == 4;
-  const int gf = tid / 32, gg = (tid / 16) % 2, gm = 1 + tid % 16;
-  R gv[NEQ];
-  unsigned gw = 0;
-  if constexpr (early) {
-    if (tid < 128) {
-      const int2 d = a.fd[li * 4 + gf];
-#pragma unroll
-      for (int k = 0; k < NEQ; ++k) gw |= unsigned(ghost_value<R>(upool, bs, a, b, d, gf, gg, gm, k, gv[k])) << k;
-    }
+  // dt, dt/dx, dt/dy and whether the block's level has viscosity, once for
+  // all its threads (read after the barriers below)
+  LeafScalars<R>& sc = leaf_scalars<R>();
+  if (tid == W2D_THREADS - 1) {
+    const int lev = a.lev[b];
+    const double dtb = step_dt(a, b, dt);
+    sc.dt = R(dtb);
+    sc.dtdx = R(dtb / geo_dx(a, b, lev));
+    sc.dtdy = R(dtb / geo_dy(a, b, lev));
+    sc.visc = lev >= (geo_nlevs(a, b) - 1);
   }
-  if (!wait_tiles_p<U>(bar, a.err, b, par)) return false;
-  if (tid < 128) {
-    int i, j;
-    ghost_ij(gf, gg, gm, i, j);
-    if constexpr (early) {
-#pragma unroll
-      for (int k = 0; k < NEQ; ++k)
-        if (gw >> k & 1u) st[k][j + 1][i + 1] = gv[k];
-    } else {
-      const int2 d = a.fd[li * 4 + gf];
-#pragma unroll
-      for (int k = 0; k < NEQ; ++k) {
-        R v;
-        if (ghost_value<R>(upool, bs, a, b, d, gf, gg, gm, k, v)) st[k][j + 1][i + 1] = v;
-      }
-    }
-  }
-  if (a.jet && a.jetblk[li]) jet_interior_fn<R, NEQ>(st, a, b, nullptr);
-  __syncthreads();
 
-  // u ghosts = up ghosts (u = up, src/tstep.f90:85; the old u stays in so),
-  // then calcprim(up) in place
+  // boundaryII and calcprim(up) in place, with u ghosts = up ghosts (u = up,
+  // src/tstep.f90:85; the old u stays in so).  Four warps gather the ghosts
+  // from the pool (box faces read the block's own interior there too) while
+  // the tiles land and convert them; the other five meanwhile convert the
+  // interior: no cell waits for another's gather.  (A gather by four warps,
+  // a barrier, then all cells in two uneven rounds: full step on 8,835 blocks
+  // 219 us, barrier stalls 3.7 per issue; so, with the leaf's scalars formed
+  // once and its statistics finished behind the last barrier: 198 us, 1.7.)
   R* __restrict__ pb = (pa.cooling == COOL_DMC) ? (R*)a.prim + (size_t)b * bs : nullptr;
-  for (int c = tid; c < W2D_CELLS; c += W2D_THREADS) {
-    const int ti = c % W2D_W, tj = c / W2D_W;
-    const bool gx = (ti < 2 || ti > 17), gy = (tj < 2 || tj > 17);
-    if (gx && gy) continue;  // corner
+  if (tid < 128) {
+    const int gf = tid / 32, gg = (tid / 16) % 2;
+    int i, j;
+    ghost_ij(gf, gg, 1 + tid % 16, i, j);
+    const int2 d = a.fd[li * 4 + gf];
     R uu[NEQ], q[NEQ], T;
+    bool w = false;
 #pragma unroll
-    for (int k = 0; k < NEQ; ++k) uu[k] = st[k][tj][ti];
-    if (gx || gy) {
+    for (int k = 0; k < NEQ; ++k) w = ghost_value<R>(upool, bs, a, b, d, gf, gg, 1 + tid % 16, k, uu[k]);
+    if (!wait_tiles_p<U>(bar, a.err, b, par)) return false;
+    if (!w) {   // a face no entry writes keeps what it has
 #pragma unroll
-      for (int k = 0; k < NEQ; ++k) u[k * W2D_CELLS + c] = uu[k];
+      for (int k = 0; k < NEQ; ++k) uu[k] = st[k][j + 1][i + 1];
     }
     uprim<NEQ>(ph, q, uu, T);
 #pragma unroll
-    for (int k = 0; k < NEQ; ++k) st[k][tj][ti] = q[k];
-    if (pb != nullptr && (ti == 0 || ti == 19 || tj == 0 || tj == 19)) {
+    for (int k = 0; k < NEQ; ++k) {
+      u[k * W2D_CELLS + cidx(i, j)] = uu[k];
+      st[k][j + 1][i + 1] = q[k];
+      if (pb != nullptr && gg == 1) pb[k * W2D_CELLS + cidx(i, j)] = q[k];
+    }
+  } else {
+    if (!wait_tiles_p<U>(bar, a.err, b, par)) return false;
+    const bool jetted = a.jet && a.jetblk[li];
+    for (int c = tid - 128; c < 256; c += W2D_THREADS - 128) {
+      const int i = 1 + c % 16, j = 1 + c / 16;
+      R uu[NEQ], q[NEQ], T;
 #pragma unroll
-      for (int k = 0; k < NEQ; ++k) pb[k * W2D_CELLS + c] = q[k];
+      for (int k = 0; k < NEQ; ++k) uu[k] = st[k][j + 1][i + 1];
+      if (jetted && in_jet(a, b, i, j)) {
+#pragma unroll
+        for (int k = 0; k < (NEQ < 6 ? NEQ : 6); ++k) uu[k] = R(a.jet_u[k]);
+      }
+      uprim<NEQ>(ph, q, uu, T);
+#pragma unroll
+      for (int k = 0; k < NEQ; ++k) st[k][j + 1][i + 1] = q[k];
     }
   }
   __syncthreads();
@@ -907,13 +955,15 @@ __device__ __forceinline__ bool full_leaf(const KArgs& a, const PhysArgs& pa, do
   if (tid < 256) {
     const int i = 1 + tid % 16, j = 1 + tid / 16;
     const int ti = i + 1, tj = j + 1;
+    const R dtdx = sc.dtdx, dtdy = sc.dtdy, eta = R(a.eta);
+    const bool visc = sc.visc != 0;
     R S[NEQ];
-    if (pa.cyl) cyl_sources<R, NEQ>(st, ti, tj, R(cyl_radius(a, b, lev, j)), ph.cv, S);
+    if (pa.cyl) cyl_sources<R, NEQ>(st, ti, tj, R(cyl_radius(a, b, a.lev[b], j)), ph.cv, S);
 #pragma unroll
     for (int k = 0; k < NEQ; ++k) {
       const R uo = so[k][tj][ti];
       R v = uo - dtdx * (sf[k][j - 1][i] - sf[k][j - 1][i - 1]) - dtdy * (sg[k][j][i - 1] - sg[k][j - 1][i - 1]);
-      if (pa.cyl) v = v + R(dtb) * S[k];   // src/step.f90:35-36, before viscosity
+      if (pa.cyl) v = v + sc.dt * S[k];   // src/step.f90:35-36, before viscosity
       if (visc)
         v = v + eta * (so[k][tj][ti + 1] + so[k][tj][ti - 1] + so[k][tj + 1][ti] + so[k][tj - 1][ti] - R(4.) * uo);
       u[k * W2D_CELLS + cidx(i, j)] = v;
@@ -924,9 +974,10 @@ __device__ __forceinline__ bool full_leaf(const KArgs& a, const PhysArgs& pa, do
     }
   }
   // the statistics of the new interior (timestep's partial, most of
-  // criteria); sf is free once every thread has passed the next barrier
-  if (a.split_stats) interior_stats<R, NEQ>(st, reinterpret_cast<double*>(&sf[0][0][0]), ph, a, b, lev);
+  // criteria)
+  if (a.split_stats) interior_stats<R, NEQ>(st, sred, ph);
   leaf_end();
+  if (a.split_stats) stats_finish<R>(sred, a, b);
   return true;
 }
 
@@ -988,9 +1039,7 @@ __device__ __forceinline__ void fill1_leaf(const KArgs& a, const PhysArgs& pa, c
   uprim<NEQ>(ph, qc, uc, T);
   const R fl = R(1e-15);
   const R am = fmaxr(fl, absr(qc[3])), am2 = fmaxr(fl, absr(qc[0]));
-  double gr = (double)fmaxr(divr(absr(qg[3] - qc[3]), am), divr(absr(qg[0] - qc[0]), am2));
-#pragma unroll
-  for (int o = 16; o > 0; o >>= 1) gr = fmax(gr, __shfl_xor_sync(0xffffffffu, gr, o));
+  const double gr = (double)warp_max0<true>(fmaxr(divr(absr(qg[3] - qc[3]), am), divr(absr(qg[0] - qc[0]), am2)));
   // the full step wrote the interior maximum; both are >= 0, so their
   // bit patterns order as the values
   if ((t & 31) == 0)
