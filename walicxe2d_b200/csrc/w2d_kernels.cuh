@@ -624,12 +624,13 @@ __device__ __forceinline__ void interior_stats(R (*st)[W2D_W][W2D_W], double* sr
   const int i = 1 + tid % 16, j = 1 + tid / 16;
   const int ti = i + 1, tj = j + 1;
   R au = R(0.), av = R(0.), rho = R(0.), p = R(0.);
+  typename DenOf<R>::T dn;
   if (tid < 256) {
     R q[NEQ], nv[NEQ], T;
 #pragma unroll
     for (int k = 0; k < NEQ; ++k) nv[k] = st[k][tj][ti];
-    uprim<NEQ>(ph, q, nv, T);
-    const R cs = sound(ph, q[3], q[0]);
+    uprim<NEQ>(ph, q, nv, T, dn);
+    const R cs = sound(ph, q[3], dn);
     au = absr(q[1]) + cs;
     av = absr(q[2]) + cs;
     rho = q[0];
@@ -642,13 +643,13 @@ __device__ __forceinline__ void interior_stats(R (*st)[W2D_W][W2D_W], double* sr
   __syncthreads();
   if (tid < 256) {
     const R fl = R(1e-15);
-    const R am = fmaxr(fl, absr(p)), am2 = fmaxr(fl, absr(rho));
+    const R am = fmaxr(fl, absr(p));   // (rho, above the same floor, is its own scale)
     R dp = R(0.), dr = R(0.);
     if (i < W2D_NX) { dp = fmaxr(dp, absr(st[3][tj][ti + 1] - p)); dr = fmaxr(dr, absr(st[0][tj][ti + 1] - rho)); }
     if (i > 1) { dp = fmaxr(dp, absr(st[3][tj][ti - 1] - p)); dr = fmaxr(dr, absr(st[0][tj][ti - 1] - rho)); }
     if (j < W2D_NX) { dp = fmaxr(dp, absr(st[3][tj + 1][ti] - p)); dr = fmaxr(dr, absr(st[0][tj + 1][ti] - rho)); }
     if (j > 1) { dp = fmaxr(dp, absr(st[3][tj - 1][ti] - p)); dr = fmaxr(dr, absr(st[0][tj - 1][ti] - rho)); }
-    const R grad = warp_max0(fmaxr(divr(dp, am), divr(dr, am2)));
+    const R grad = warp_max0(fmaxr(divr(dp, am), quot(dr, dn)));
     au = warp_max0(au);
     av = warp_max0(av);
     if ((tid & 31) == 0) {
@@ -713,8 +714,15 @@ __device__ __forceinline__ double cyl_radius(const KArgs& a, int b, int lev, int
 template <typename R, int NEQ>
 __host__ __device__ constexpr size_t smem_half()
 {
-  return 128 + sizeof(R) * (2 * NEQ * W2D_CELLS + W2D_CELLS + 2 * NEQ * 272);
+  return 128 + sizeof(R) * ((2 * NEQ + 1 + (sizeof(R) == 4)) * W2D_CELLS + 2 * NEQ * 272);
 }
+
+// the density rho as a divisor, its reciprocal read back in FP32
+__device__ __forceinline__ Den64 kept_den(double rho, const double*) { return {rho}; }
+__device__ __forceinline__ Den32 kept_den(float, const float* y) { return {*y}; }
+// one of two densities as a divisor (rho: the one chosen)
+__device__ __forceinline__ Den64 either(const Den64&, const Den64&, bool, double rho) { return {rho}; }
+__device__ __forceinline__ Den32 either(const Den32& l, const Den32& r, bool left, float) { return {left ? l.y : r.y}; }
 
 // One leaf of the half step (position li of the leaf list); the tile
 // barrier completes with phase parity `par`.  Returns false when the tile
@@ -723,13 +731,17 @@ template <typename R, int NEQ, int SOLVER, bool U = false>
 __device__ __forceinline__ bool half_leaf(const KArgs& a, const PhysArgs& pa, double dt, int li, uint32_t par)
 {
   // su: the tile as loaded (u, or the stored primitives under DMC); st:
-  // the primitives of cells 0..17; scs: their sound speeds
+  // the primitives of cells 0..17; scs: their sound speeds; siv
+  // (FP32): the reciprocals of their densities
   uint64_t* bar = reinterpret_cast<uint64_t*>(w2d_smem);
   R(*su)[W2D_W][W2D_W] = reinterpret_cast<R(*)[W2D_W][W2D_W]>(w2d_smem + 128);
   R(*st)[W2D_W][W2D_W] = reinterpret_cast<R(*)[W2D_W][W2D_W]>(w2d_smem + 128 + sizeof(R) * NEQ * W2D_CELLS);
   R(*scs)[W2D_W] = reinterpret_cast<R(*)[W2D_W]>(w2d_smem + 128 + sizeof(R) * 2 * NEQ * W2D_CELLS);
-  R(*sf)[16][17] = reinterpret_cast<R(*)[16][17]>(w2d_smem + 128 + sizeof(R) * (2 * NEQ + 1) * W2D_CELLS);
-  R(*sg)[17][16] = reinterpret_cast<R(*)[17][16]>(w2d_smem + 128 + sizeof(R) * ((2 * NEQ + 1) * W2D_CELLS + NEQ * 272));
+  R(*siv)[W2D_W] = reinterpret_cast<R(*)[W2D_W]>(w2d_smem + 128 + sizeof(R) * (2 * NEQ + 1) * W2D_CELLS);
+  constexpr bool inv = sizeof(R) == 4;
+  constexpr int NT = 2 * NEQ + 1 + inv;   // tiles
+  R(*sf)[16][17] = reinterpret_cast<R(*)[16][17]>(w2d_smem + 128 + sizeof(R) * NT * W2D_CELLS);
+  R(*sg)[17][16] = reinterpret_cast<R(*)[17][16]>(w2d_smem + 128 + sizeof(R) * (NT * W2D_CELLS + NEQ * 272));
   const Phys<R> ph = make_phys<R, SOLVER, -1>(pa);
   const int tid = threadIdx.x;
   const size_t bs = (size_t)NEQ * W2D_CELLS;
@@ -760,15 +772,19 @@ __device__ __forceinline__ bool half_leaf(const KArgs& a, const PhysArgs& pa, do
     R q[NEQ];
 #pragma unroll
     for (int k = 0; k < NEQ; ++k) q[k] = su[k][tj][ti];
+    typename DenOf<R>::T dn;
     if (!dmc) {
       R uu[NEQ], T;
 #pragma unroll
       for (int k = 0; k < NEQ; ++k) uu[k] = q[k];
-      uprim<NEQ>(ph, q, uu, T);
+      uprim<NEQ>(ph, q, uu, T, dn);
+    } else {
+      dn = den(q[0]);
     }
 #pragma unroll
     for (int k = 0; k < NEQ; ++k) st[k][tj][ti] = q[k];
-    scs[tj][ti] = sound(ph, q[3], q[0]);
+    scs[tj][ti] = sound(ph, q[3], dn);
+    if constexpr (inv) siv[tj][ti] = dn.y;
   }
   __syncthreads();
 
@@ -778,7 +794,8 @@ __device__ __forceinline__ bool half_leaf(const KArgs& a, const PhysArgs& pa, do
       const int i = tid % 17, j = 1 + tid / 17;
 #pragma unroll
       for (int k = 0; k < NEQ; ++k) { pl[k] = st[k][j + 1][i + 1]; pr[k] = st[k][j + 1][i + 2]; }
-      if (!riemann<NEQ>(ph, pl, pr, scs[j + 1][i + 1], scs[j + 1][i + 2], ff)) set_err(a.err, ERR_HLLC, b, i, j);
+      if (!riemann<NEQ>(ph, pl, pr, scs[j + 1][i + 1], scs[j + 1][i + 2],
+                        [&](bool left, R rho) { return kept_den(rho, &siv[j + 1][left ? i + 1 : i + 2]); }, ff)) set_err(a.err, ERR_HLLC, b, i, j);
 #pragma unroll
       for (int k = 0; k < NEQ; ++k) sf[k][j - 1][i] = ff[k];
     }
@@ -788,7 +805,8 @@ __device__ __forceinline__ bool half_leaf(const KArgs& a, const PhysArgs& pa, do
       for (int k = 0; k < NEQ; ++k) { pl[k] = st[k][j + 1][i + 1]; pr[k] = st[k][j + 2][i + 1]; }
       R t = pl[1]; pl[1] = pl[2]; pl[2] = t;
       t = pr[1]; pr[1] = pr[2]; pr[2] = t;
-      if (!riemann<NEQ>(ph, pl, pr, scs[j + 1][i + 1], scs[j + 2][i + 1], ff)) set_err(a.err, ERR_HLLC, b, i, j);
+      if (!riemann<NEQ>(ph, pl, pr, scs[j + 1][i + 1], scs[j + 2][i + 1],
+                        [&](bool left, R rho) { return kept_den(rho, &siv[left ? j + 1 : j + 2][i + 1]); }, ff)) set_err(a.err, ERR_HLLC, b, i, j);
       t = ff[1]; ff[1] = ff[2]; ff[2] = t;
 #pragma unroll
       for (int k = 0; k < NEQ; ++k) sg[k][j][i - 1] = ff[k];
@@ -925,8 +943,10 @@ __device__ __forceinline__ bool full_leaf(const KArgs& a, const PhysArgs& pa, do
         prr[k] = st[k][j + 1][i + 3];
         limit1<R>(ph.limiter, pll[k], pl[k], pr[k], prr[k]);
       }
-      R csl = sound(ph, pl[3], pl[0]), csr = sound(ph, pr[3], pr[0]);
-      if (!riemann<NEQ>(ph, pl, pr, csl, csr, ff)) set_err(a.err, ERR_HLLC, b, i, j);
+      const typename DenOf<R>::T dl = den(pl[0]), dr = den(pr[0]);
+      const R csl = sound(ph, pl[3], dl), csr = sound(ph, pr[3], dr);
+      if (!riemann<NEQ>(ph, pl, pr, csl, csr, [&](bool left, R rho) { return either(dl, dr, left, rho); }, ff))
+        set_err(a.err, ERR_HLLC, b, i, j);
 #pragma unroll
       for (int k = 0; k < NEQ; ++k) sf[k][j - 1][i] = ff[k];
     }
@@ -942,8 +962,10 @@ __device__ __forceinline__ bool full_leaf(const KArgs& a, const PhysArgs& pa, do
       }
       R t = pl[1]; pl[1] = pl[2]; pl[2] = t;
       t = pr[1]; pr[1] = pr[2]; pr[2] = t;
-      R csl = sound(ph, pl[3], pl[0]), csr = sound(ph, pr[3], pr[0]);
-      if (!riemann<NEQ>(ph, pl, pr, csl, csr, ff)) set_err(a.err, ERR_HLLC, b, i, j);
+      const typename DenOf<R>::T dl = den(pl[0]), dr = den(pr[0]);
+      const R csl = sound(ph, pl[3], dl), csr = sound(ph, pr[3], dr);
+      if (!riemann<NEQ>(ph, pl, pr, csl, csr, [&](bool left, R rho) { return either(dl, dr, left, rho); }, ff))
+        set_err(a.err, ERR_HLLC, b, i, j);
       t = ff[1]; ff[1] = ff[2]; ff[2] = t;
 #pragma unroll
       for (int k = 0; k < NEQ; ++k) sg[k][j][i - 1] = ff[k];
