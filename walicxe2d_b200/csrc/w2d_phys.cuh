@@ -31,6 +31,12 @@ __device__ __forceinline__ float absr(float x) { return fabsf(x); }
 __device__ __forceinline__ double signr(double a) { return copysign(1.0, a); }
 __device__ __forceinline__ float signr(float a) { return copysignf(1.0f, a); }
 
+// y + x/2 and y - x/2 (halving is exact, so one operation rounds as two)
+__device__ __forceinline__ double add_half(double y, double x) { return fma(0.5, x, y); }
+__device__ __forceinline__ double sub_half(double y, double x) { return fma(-0.5, x, y); }
+__device__ __forceinline__ float add_half(float y, float x) { return y + 0.5f * x; }
+__device__ __forceinline__ float sub_half(float y, float x) { return y - 0.5f * x; }
+
 enum { SOLVER_HLLC = 0, SOLVER_HLL = 1, SOLVER_HLL_HLLC = 2 };
 enum { COOL_NONE = 0, COOL_H = 1, COOL_DMC = 2 };
 
@@ -111,7 +117,7 @@ __device__ __forceinline__ void uprim(const Phys<R>& ph, R* prim, const R* uu, R
   prim[2] = quot(uu[2], dn);
 #pragma unroll
   for (int k = 4; k < NEQ; ++k) prim[k] = uu[k];
-  prim[3] = div_cv(ph, uu[3] - R(0.5) * r * (prim[1] * prim[1] + prim[2] * prim[2]));
+  prim[3] = div_cv(ph, sub_half(uu[3], r * (prim[1] * prim[1] + prim[2] * prim[2])));
   prim[3] = fmaxr(prim[3], tiny);
   if (ph.cooling == COOL_NONE) {
     T = quot(prim[3], dn);
@@ -139,7 +145,7 @@ __device__ __forceinline__ void primu(const Phys<R>& ph, const R* p, R* uu)
   uu[0] = p[0];
   uu[1] = p[0] * p[1];
   uu[2] = p[0] * p[2];
-  uu[3] = R(0.5) * p[0] * (p[1] * p[1] + p[2] * p[2]) + ph.cv * p[3];
+  uu[3] = add_half(ph.cv * p[3], p[0] * (p[1] * p[1] + p[2] * p[2]));
 #pragma unroll
   for (int k = 4; k < NEQ; ++k) uu[k] = p[k];
 }
@@ -148,7 +154,7 @@ __device__ __forceinline__ void primu(const Phys<R>& ph, const R* p, R* uu)
 template <int NEQ, typename R>
 __device__ __forceinline__ void primf(const Phys<R>& ph, const R* p, R* ff)
 {
-  R etot = R(0.5) * p[0] * (p[1] * p[1] + p[2] * p[2]) + ph.cv * p[3];
+  R etot = add_half(ph.cv * p[3], p[0] * (p[1] * p[1] + p[2] * p[2]));
   ff[0] = p[0] * p[1];
   ff[1] = p[0] * p[1] * p[1] + p[3];
   ff[2] = p[0] * p[1] * p[2];
@@ -176,13 +182,12 @@ __device__ __forceinline__ void hllc_star(const Phys<R>& ph, const R* q, R s, R 
   // component by component (fewer values live at once), each term formed as
   // primf, primu and the star state form it: F + s (U* - U)
   const R rhost = divr(q[0] * smus, s - sst);
-  const R ek = R(0.5) * q[0] * (q[1] * q[1] + q[2] * q[2]) + ph.cv * q[3];
+  const R ek = add_half(ph.cv * q[3], q[0] * (q[1] * q[1] + q[2] * q[2]));
   ff[0] = q[0] * q[1] + s * (rhost - q[0]);
   ff[1] = (q[0] * q[1] * q[1] + q[3]) + s * (rhost * sst - q[0] * q[1]);
   ff[2] = q[0] * q[1] * q[2] + s * (rhost * q[2] - q[0] * q[2]);
-  const R etot = R(0.5) * q[0] * (q[1] * q[1] + q[2] * q[2]) + ph.cv * q[3];
-  ff[3] = q[1] * (etot + q[3]) +
-          s * (rhost * (quot(ek, dn) + (sst - q[1]) * (sst + divr(q[3], den * smus))) - etot);
+  ff[3] = q[1] * (ek + q[3]) +
+          s * (rhost * (quot(ek, dn) + (sst - q[1]) * (sst + divr(q[3], den * smus))) - ek);
 #pragma unroll
   for (int k = 4; k < NEQ; ++k) ff[k] = q[k] * q[1] + s * (quot(rhost * q[k], dn) - q[k]);
 }
@@ -258,6 +263,24 @@ __device__ __forceinline__ bool riemann(const Phys<R>& ph, R* pl, const R* pr, R
   return true;
 }
 
+// s max(0, min(|a|, s b)) with s = sign(a) (minmod).  In FP64 the signs move
+// as bits instead of through two multiplications, and the zero comes from
+// the sign of the minimum instead of a comparison (a minimum between -2^-1042
+// and 0 stays: no cell value feels it).
+__device__ __forceinline__ double minmod(double a, double b)
+{
+  const unsigned s = (unsigned)__double2hiint(a) & 0x80000000u;
+  const double sb = __hiloint2double(__double2hiint(b) ^ (int)s, __double2loint(b));
+  const double m = fminr(fabs(a), sb);
+  const bool neg = (unsigned)__double2hiint(m) > 0x80000000u;
+  return __hiloint2double(neg ? (int)s : __double2hiint(m) ^ (int)s, neg ? 0 : __double2loint(m));
+}
+__device__ __forceinline__ float minmod(float a, float b)
+{
+  const float s = signr(a);
+  return s * fmaxr(0.f, fminr(absr(a), s * b));
+}
+
 // average(a,b) of src/limiter.f90:24-86 for LIMITER = -1..6
 template <typename R>
 __device__ __forceinline__ R average(int limiter, R a, R b)
@@ -265,7 +288,7 @@ __device__ __forceinline__ R average(int limiter, R a, R b)
   switch (limiter) {
     case -1: return R(0.);
     case 0: return R(0.5) * (a + b);
-    case 1: { R s = signr(a); return s * fmaxr(R(0.), fminr(absr(a), s * b)); }
+    case 1: return minmod(a, b);
     case 2:
       if (a * b <= R(0.)) return R(0.);
       return divr(a * b * (a + b), a * a + b * b);
@@ -304,8 +327,8 @@ __device__ __forceinline__ void limit1(int limiter, R pll, R& pl, R& pr, R prr)
   R dr = prr - pr;
   R al = average<R>(limiter, dl, dm);
   R ar = average<R>(limiter, dm, dr);
-  pl = pl + al * R(0.5);
-  pr = pr - ar * R(0.5);
+  pl = add_half(pl, al);
+  pr = sub_half(pr, ar);
 }
 
 }  // namespace w2d
