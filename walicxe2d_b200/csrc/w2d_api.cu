@@ -108,10 +108,20 @@ struct Shape {
 constexpr Shape kShapes[] = {{0, 0}, {2, 0}, {4, 0}, {4, 1}, {8, 0}, {8, 1}};
 constexpr int kNShape = (int)(sizeof(kShapes) / sizeof(kShapes[0]));
 
+// CTAs per SM of a shape's persistent grid.  The cooling kernel holds three
+// per SM (64 registers, 320 threads): its grids of 4 and 8 would leave the
+// last wave a third full (FP32 ensemble of 6,641 leaves: 151 us on 4 per SM,
+// 130 on 3; compiled for 2 per SM 137).
+int shape_per_sm(int sh, int tk)
+{
+  const int per = kShapes[sh].per_sm;
+  return tk == TK_COOL && per >= 4 ? per * 3 / 4 : per;
+}
+
 void apply_shape(W2dCtx* c, KArgs& a, int tk)
 {
   const int sh = c->tune_left > 0 ? c->tune_cur : c->tshape[tk];
-  a.grid = kShapes[sh].per_sm * c->nsm;
+  a.grid = shape_per_sm(sh, tk) * c->nsm;
   a.sched = kShapes[sh].sched;
 }
 
@@ -2036,7 +2046,7 @@ int w2d_tuning(W2dCtx* c, int32_t* shape, double* ms, int* tuning_left)
     const int sh = c->tshape[k];
     if (shape) {
       shape[3 * k] = sh;
-      shape[3 * k + 1] = kShapes[sh].per_sm;
+      shape[3 * k + 1] = shape_per_sm(sh, k);
       shape[3 * k + 2] = kShapes[sh].sched;
     }
     if (ms) ms[k] = c->tune_n[k][sh] > 0 ? c->tune_ms[k][sh] / c->tune_n[k][sh] : 0.0;
