@@ -237,7 +237,7 @@ __host__ __device__ constexpr size_t smem_cool()
 
 // Threads of the cooling kernel: one per cell 0..17 x 0..17 of a block
 // without its four corners (320), so the FP64 routine runs in one round;
-// the block statistics use the first 256 (warps 8 and 9 add neutral values).
+// the block statistics use the first 256, and warp 8 combines them.
 constexpr int W2D_COOL_THREADS = 320;
 
 template <typename R, int NEQ, bool P>
@@ -303,8 +303,9 @@ __global__ void __launch_bounds__(W2D_COOL_THREADS, 3) k_cool(KArgs a, PhysArgs 
     }
   }
   __syncthreads();
-  block_stats<R, NEQ>(st, ph, a, pa, b, sred);
+  block_stats<R, NEQ>(st, ph, a, pa, sred);
   leaf_end();
+  stats_finish<R>(sred, a, b, pa.cooling == COOL_DMC);
   }
 }
 

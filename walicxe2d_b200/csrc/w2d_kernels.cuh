@@ -541,67 +541,78 @@ __device__ __forceinline__ float warp_max0(float x)
 //   min_c RN(dx/(|u|+cs)_c) = RN(dx / max_c (|u|+cs)_c)
 //   max_n RN(|dp_n|/am)     = RN(max_n |dp_n| / am)
 // exactly, and the results equal the reference's.
+//
+// The warps' extrema go to sred; stats_finish combines them after the
+// next CTA barrier in the warp behind the 256 cells' threads, while the
+// others go on.
 template <typename R, int NEQ>
 __device__ __forceinline__ void block_stats(const R (*sp)[W2D_W][W2D_W], const Phys<R>& ph, const KArgs& a,
-                                            const PhysArgs& pa, int b, double* sred)
+                                            const PhysArgs& pa, double* sred)
 {
   const int tid = threadIdx.x;
-  R au = R(0.), av = R(0.), grad = R(0.);
+  if (tid >= 256) return;
+  const int i = 1 + tid % 16, j = 1 + tid / 16;
+  const int ti = i + 1, tj = j + 1;
+  const R rho = sp[0][tj][ti], vx = sp[1][tj][ti], vy = sp[2][tj][ti], p = sp[3][tj][ti];
+  const typename DenOf<R>::T dn = den(rho);
+  const R cs = sound(ph, p, dn);
+  const R au = warp_max0(absr(vx) + cs), av = warp_max0(absr(vy) + cs);
+  const R am = fmaxr(R(1e-15), absr(p));   // (rho, above the same floor, is its own scale)
+  R dp = absr(sp[3][tj][ti + 1] - p);
+  dp = fmaxr(dp, absr(sp[3][tj][ti - 1] - p));
+  dp = fmaxr(dp, absr(sp[3][tj + 1][ti] - p));
+  dp = fmaxr(dp, absr(sp[3][tj - 1][ti] - p));
+  R dr = absr(sp[0][tj][ti + 1] - rho);
+  dr = fmaxr(dr, absr(sp[0][tj][ti - 1] - rho));
+  dr = fmaxr(dr, absr(sp[0][tj + 1][ti] - rho));
+  dr = fmaxr(dr, absr(sp[0][tj - 1][ti] - rho));
+  const R grad = warp_max0(fmaxr(divr(dp, am), quot(dr, dn)));
   double dtc = 1e30;
-  if (tid < 256) {
-    const int i = 1 + tid % 16, j = 1 + tid / 16;
-    const int ti = i + 1, tj = j + 1;
-    const R rho = sp[0][tj][ti], vx = sp[1][tj][ti], vy = sp[2][tj][ti], p = sp[3][tj][ti];
-    const R cs = sound(ph, p, rho);
-    au = absr(vx) + cs;
-    av = absr(vy) + cs;
-    const R fl = R(1e-15);
-    const R am = fmaxr(fl, absr(p)), am2 = fmaxr(fl, absr(rho));
-    R dp = absr(sp[3][tj][ti + 1] - p);
-    dp = fmaxr(dp, absr(sp[3][tj][ti - 1] - p));
-    dp = fmaxr(dp, absr(sp[3][tj + 1][ti] - p));
-    dp = fmaxr(dp, absr(sp[3][tj - 1][ti] - p));
-    R dr = absr(sp[0][tj][ti + 1] - rho);
-    dr = fmaxr(dr, absr(sp[0][tj][ti - 1] - rho));
-    dr = fmaxr(dr, absr(sp[0][tj + 1][ti] - rho));
-    dr = fmaxr(dr, absr(sp[0][tj - 1][ti] - rho));
-    grad = fmaxr(divr(dp, am), divr(dr, am2));
-    if (pa.cooling == COOL_DMC) {                    // src/timestep.f90:34-41
-      const double T = ((double)p / (double)rho) * pa.tempsc;
-      if (T > 1e4) {
-        const double aloss = d_cooldmc(a.cooltab, T) * ((double)rho * (double)rho);
-        dtc = pa.cv * (double)p / aloss;
-      }
+  if (pa.cooling == COOL_DMC) {                    // src/timestep.f90:34-41
+    const double T = ((double)p / (double)rho) * pa.tempsc;
+    if (T > 1e4) {
+      const double aloss = d_cooldmc(a.cooltab, T) * ((double)rho * (double)rho);
+      dtc = pa.cv * (double)p / aloss;
     }
-  }
-  au = warp_max0(au);
-  av = warp_max0(av);
-  grad = warp_max0(grad);
-  if (pa.cooling == COOL_DMC) {
 #pragma unroll
     for (int o = 16; o > 0; o >>= 1) dtc = fmin(dtc, __shfl_xor_sync(0xffffffffu, dtc, o));
   }
   if ((tid & 31) == 0) {
     sred[tid >> 5] = (double)au;
-    sred[16 + (tid >> 5)] = (double)av;
-    sred[32 + (tid >> 5)] = (double)grad;
-    sred[48 + (tid >> 5)] = dtc;
+    sred[8 + (tid >> 5)] = (double)av;
+    sred[16 + (tid >> 5)] = (double)grad;
+    sred[24 + (tid >> 5)] = dtc;
   }
-  __syncthreads();
-  if (tid == 0) {
-    double m0 = sred[0], m1 = sred[16], m2 = sred[32], m3 = sred[48];
-    for (int w = 1; w < W2D_THREADS / 32; ++w) {
-      m0 = fmax(m0, sred[w]);
-      m1 = fmax(m1, sred[16 + w]);
-      m2 = fmax(m2, sred[32 + w]);
-      m3 = fmin(m3, sred[48 + w]);
-    }
+}
+
+// The maxima of the eight warps that have cells, in warp 8: the block's CFL
+// partial and criteria maximum (and DMC limit, when dmc)
+template <typename R>
+__device__ __forceinline__ void stats_finish(const double* sred, const KArgs& a, int b, bool dmc = false)
+{
+  const int lane = (int)threadIdx.x - 256;
+  if (lane < 0 || lane >= 32) return;
+  double m0 = 0., m1 = 0., m2 = 0., m3 = 1e30;
+  if (lane < 8) {
+    m0 = sred[lane];
+    m1 = sred[8 + lane];
+    m2 = sred[16 + lane];
+    if (dmc) m3 = sred[24 + lane];
+  }
+  m0 = warp_max0(m0);
+  m1 = warp_max0(m1);
+  m2 = warp_max0(m2);
+  if (dmc) {
+#pragma unroll
+    for (int o = 4; o > 0; o >>= 1) m3 = fmin(m3, __shfl_xor_sync(0xffffffffu, m3, o));
+  }
+  if (lane == 0) {
     const int lev = a.lev[b];
     const R t1 = R(geo_dx(a, b, lev)) / R(m0);
     const R t2 = R(geo_dy(a, b, lev)) / R(m1);
     a.cfl[b] = (double)fminr(t1, t2);
     a.grad[b] = m2;
-    if (pa.cooling == COOL_DMC) a.dtcool[b] = m3;
+    if (dmc) a.dtcool[b] = m3;
   }
 }
 
@@ -657,29 +668,6 @@ __device__ __forceinline__ void interior_stats(R (*st)[W2D_W][W2D_W], double* sr
       sred[8 + (tid >> 5)] = (double)av;
       sred[16 + (tid >> 5)] = (double)grad;
     }
-  }
-}
-
-template <typename R>
-__device__ __forceinline__ void stats_finish(const double* sred, const KArgs& a, int b)
-{
-  const int lane = (int)threadIdx.x - 256;
-  if (lane < 0) return;
-  double m0 = 0., m1 = 0., m2 = 0.;
-  if (lane < 8) {
-    m0 = sred[lane];
-    m1 = sred[8 + lane];
-    m2 = sred[16 + lane];
-  }
-  m0 = warp_max0(m0);
-  m1 = warp_max0(m1);
-  m2 = warp_max0(m2);
-  if (lane == 0) {
-    const int lev = a.lev[b];
-    const R t1 = R(geo_dx(a, b, lev)) / R(m0);
-    const R t2 = R(geo_dy(a, b, lev)) / R(m1);
-    a.cfl[b] = (double)fminr(t1, t2);
-    a.grad[b] = m2;
   }
 }
 
@@ -1145,8 +1133,9 @@ __global__ void __launch_bounds__(W2D_THREADS, w2d_minb<R>(P)) k_calcprim(KArgs 
     }
   }
   __syncthreads();
-  block_stats<R, NEQ>(st, ph, a, pa, b, sred);
+  block_stats<R, NEQ>(st, ph, a, pa, sred);
   leaf_end();
+  stats_finish<R>(sred, a, b, pa.cooling == COOL_DMC);
   }
 }
 
@@ -1299,7 +1288,9 @@ __global__ void __launch_bounds__(W2D_THREADS) k_amr(KArgs a, PhysArgs pa, const
     }
   }
   __syncthreads();
-  block_stats<R, NEQ>(st, ph, a, pa, b, sred);
+  block_stats<R, NEQ>(st, ph, a, pa, sred);
+  __syncthreads();
+  stats_finish<R>(sred, a, b, pa.cooling == COOL_DMC);
 }
 
 // pool <-> staging (block-major, FP64 as the C-ABI's host arrays) copies;
