@@ -521,9 +521,10 @@ int half_step(W2dCtx* c, double dt, const double* dt_dev)
 // ---------------------------------------------------------------------------
 // the split timestep/tstep of w2d_internal.h
 
-// src/timestep.f90:7-61 as one reduction kernel; dt stays in device memory
-// and is copied, with the error word, to pinned memory behind it
-int ctx_dt_reduce(W2dCtx* c, double** dt_dev)
+// src/timestep.f90:7-61 as one reduction kernel; dt stays in device memory,
+// and the kernel stores it, with the error word, to pinned memory where pub
+// says so
+static int dt_reduce(W2dCtx* c, const DtPublish& pub)
 {
   if (!c->have_topology) return set_error(c, W2D_ERR_STATE, 0, 0, 0, "w2d_set_topology first");
   int rc0 = ensure_leaf_list(c);
@@ -533,8 +534,14 @@ int ctx_dt_reduce(W2dCtx* c, double** dt_dev)
   int rc = launch(c, "timestep", [&] {
     return launch_dt(c->d_leaves, nl, dev ? c->d_nleaf : nullptr, dev ? 2 * c->nsm : 0, c->d_cfl, c->d_dtcool,
                      c->p.cooling == W2D_COOLINGDMC, c->p.cfl, c->p.psc, c->p.tsc, c->d_dtwork, c->d_dtcount,
-                     c->d_dt, c->st);
+                     c->d_dt, pub, c->st);
   });
+  return rc;
+}
+
+int ctx_dt_reduce(W2dCtx* c, double** dt_dev)
+{
+  int rc = dt_reduce(c, DtPublish{});
   if (dt_dev) *dt_dev = c->d_dt;
   return rc;
 }
@@ -549,8 +556,10 @@ int ctx_dt_publish(W2dCtx* c)
 
 int ctx_dt_launch(W2dCtx* c)
 {
-  int rc = ctx_dt_reduce(c, nullptr);
-  return rc ? rc : ctx_dt_publish(c);
+  int rc = dt_reduce(c, DtPublish{c->h_small, c->h_err, c->d_err});
+  if (rc) return rc;
+  if (!c->capturing) CK(cudaEventRecord(c->ev_dt, c->st));
+  return W2D_OK;
 }
 
 int ctx_half_step(W2dCtx* c)
@@ -1769,11 +1778,10 @@ int ctx_ens_dt_launch(W2dCtx* c)
 {
   int rc = launch(c, "timestep", [&] {
     return launch_dt_runs(c->d_leaves, c->d_loff, c->nruns, c->d_cfl, c->d_dtcool,
-                          c->p.cooling == W2D_COOLINGDMC, c->p.cfl, c->p.psc, c->p.tsc, c->d_dt_run, c->st);
+                          c->p.cooling == W2D_COOLINGDMC, c->p.cfl, c->p.psc, c->p.tsc, c->d_dt_run,
+                          DtPublish{c->h_dt_run, c->h_err, c->d_err}, c->st);
   });
-  if (rc) return rc;
-  CK(cudaMemcpyAsync(c->h_dt_run, c->d_dt_run, sizeof(double) * (size_t)c->nruns, cudaMemcpyDeviceToHost, c->st));
-  return W2D_OK;
+  return rc;
 }
 
 const double* ctx_ens_dt(W2dCtx* c) { return c->h_dt_run; }

@@ -15,14 +15,14 @@
 // computes exactly what w2d_timestep followed by w2d_tstep computes: the
 // half step reads the dt that k_dt left in device memory, the host reads
 // the same value back before the full step.
-int ctx_dt_launch(W2dCtx* c);                           // k_dt; dt and error word copied to pinned memory
+int ctx_dt_launch(W2dCtx* c);                           // k_dt; dt and error word stored to pinned memory
 int ctx_half_step(W2dCtx* c);                           // k_half, dt from device memory
 int ctx_dt_wait(W2dCtx* c, double* dt);                 // waits for the copy, checks the error word
 int ctx_tstep_rest(W2dCtx* c, double time, double dt);  // full step, boundaryI, prim/cooling
 // the same sequence with room for an exchange between its parts (a block
 // partition of one run over several GPUs):
 //   ctx_dt_launch  = ctx_dt_reduce (k_dt into device memory, *dt_dev its
-//                    address) + ctx_dt_publish (the copies behind it)
+//                    address) + ctx_dt_publish (copies to pinned memory)
 //   ctx_tstep_rest = ctx_full_step (boundaryII inside the full step's
 //                    gather, full step, u = up) + ctx_tstep_tail (boundaryI,
 //                    prim/cooling)

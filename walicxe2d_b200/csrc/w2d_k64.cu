@@ -8,17 +8,29 @@ namespace w2d {
 
 const Launchers& launchers64() { return k64::table; }
 
+// dt of run r, and with run 0 the error word, to the host's pinned copies
+__device__ __forceinline__ void publish_dt(const DtPublish& p, int r, double dt)
+{
+  if (!p.dt_host) return;
+  p.dt_host[r] = dt;
+  if (r == 0)
+    for (int k = 0; k < 4; ++k) p.err_host[k] = p.err[k];
+}
+
 // src/timestep.f90:48: dt = min(cfl*dtp, 0.4*dtcool*Psc/tsc), dtp and dtcool
 // the minima of the per-block partials over the leaves.  Each CTA reduces
 // 256 leaves and folds its minima into work[0..1] with 64-bit atomicMin on
 // the bit patterns (for non-negative doubles the integer order is the
-// numeric order); the last CTA to finish forms dt and resets work/count.
+// numeric order); the last CTA to finish forms dt and resets work/count.  It
+// also stores dt and the error word to the host's pinned copies (pub), in
+// place of two copies between this kernel and the half step.
 __global__ void __launch_bounds__(256) k_dt(const int* __restrict__ leaves, int n, const int* __restrict__ n_dev,
                                             const double* __restrict__ cfl,
                                             const double* __restrict__ dtcool, int use_cool,
                                             double courant, double psc, double tsc,
                                             unsigned long long* __restrict__ work,
-                                            unsigned int* __restrict__ count, double* __restrict__ dt_out)
+                                            unsigned int* __restrict__ count, double* __restrict__ dt_out,
+                                            DtPublish pub)
 {
   __shared__ double s0[8], s1[8];
   __shared__ bool last;
@@ -52,7 +64,9 @@ __global__ void __launch_bounds__(256) k_dt(const int* __restrict__ leaves, int 
     const double d1 = __longlong_as_double((long long)atomicAdd(&work[1], 0ull));
     const double a = courant * d0;
     const double c = 0.4 * d1 * psc / tsc;
-    dt_out[0] = (a < c) ? a : c;
+    const double dt = (a < c) ? a : c;
+    dt_out[0] = dt;
+    publish_dt(pub, 0, dt);
     work[0] = work[1] = (unsigned long long)__double_as_longlong(1.e30);
     *count = 0u;
   }
@@ -66,7 +80,7 @@ __global__ void __launch_bounds__(256) k_dt_runs(const int* __restrict__ leaves,
                                                  const double* __restrict__ cfl,
                                                  const double* __restrict__ dtcool, int use_cool,
                                                  double courant, double psc, double tsc,
-                                                 double* __restrict__ dt_run)
+                                                 double* __restrict__ dt_run, DtPublish pub)
 {
   __shared__ double s0[8], s1[8];
   const int r = blockIdx.x;
@@ -89,15 +103,18 @@ __global__ void __launch_bounds__(256) k_dt_runs(const int* __restrict__ leaves,
     for (int w = 1; w < 8; ++w) { m0 = fmin(m0, s0[w]); m1 = fmin(m1, s1[w]); }
     const double a = courant * m0;
     const double c = 0.4 * m1 * psc / tsc;
-    dt_run[r] = (a < c) ? a : c;
+    const double dt = (a < c) ? a : c;
+    dt_run[r] = dt;
+    publish_dt(pub, r, dt);
   }
 }
 
 cudaError_t launch_dt_runs(const int* leaves, const int* loff, int nruns, const double* cfl, const double* dtcool,
-                           int use_cool, double courant, double psc, double tsc, double* dt_run, cudaStream_t st)
+                           int use_cool, double courant, double psc, double tsc, double* dt_run, const DtPublish& pub,
+                           cudaStream_t st)
 {
   if (nruns == 0) return cudaSuccess;
-  k_dt_runs<<<nruns, 256, 0, st>>>(leaves, loff, cfl, dtcool, use_cool, courant, psc, tsc, dt_run);
+  k_dt_runs<<<nruns, 256, 0, st>>>(leaves, loff, cfl, dtcool, use_cool, courant, psc, tsc, dt_run, pub);
   return cudaGetLastError();
 }
 
@@ -137,10 +154,10 @@ cudaError_t launch_gather_leaf(const int* leaves, int n, const int* n_dev, const
 
 cudaError_t launch_dt(const int* leaves, int n, const int* n_dev, int grid, const double* cfl, const double* dtcool,
                       int use_cool, double courant, double psc, double tsc, unsigned long long* work,
-                      unsigned int* count, double* dt_out, cudaStream_t st)
+                      unsigned int* count, double* dt_out, const DtPublish& pub, cudaStream_t st)
 {
   if (grid <= 0) grid = n > 0 ? (n + 255) / 256 : 1;
-  k_dt<<<grid, 256, 0, st>>>(leaves, n, n_dev, cfl, dtcool, use_cool, courant, psc, tsc, work, count, dt_out);
+  k_dt<<<grid, 256, 0, st>>>(leaves, n, n_dev, cfl, dtcool, use_cool, courant, psc, tsc, work, count, dt_out, pub);
   return cudaGetLastError();
 }
 

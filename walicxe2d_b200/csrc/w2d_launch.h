@@ -37,17 +37,26 @@ struct Launchers {
 const Launchers& launchers64();
 const Launchers& launchers32();
 
+// Where the dt reduction leaves dt (per run) and the error word for the host:
+// pinned memory that the kernel stores to (dt_host null: nowhere).
+struct DtPublish {
+  double* dt_host;
+  int* err_host;
+  const int* err;
+};
+
 // work: two 64-bit words holding the bit pattern of 1e30; count: zero.
 // Both are restored by the kernel for the next call.
 // n_dev: leaf count in device memory (then grid > 0 is the CTA count); with
 // grid <= 0 one CTA per 256 leaves
 cudaError_t launch_dt(const int* leaves, int n, const int* n_dev, int grid, const double* cfl, const double* dtcool,
                       int use_cool, double courant, double psc, double tsc, unsigned long long* work,
-                      unsigned int* count, double* dt_out, cudaStream_t st);
+                      unsigned int* count, double* dt_out, const DtPublish& pub, cudaStream_t st);
 
 // dt_run[r] for every run of an ensemble; leaves of run r at loff[r]..loff[r+1]-1
 cudaError_t launch_dt_runs(const int* leaves, const int* loff, int nruns, const double* cfl, const double* dtcool,
-                           int use_cool, double courant, double psc, double tsc, double* dt_run, cudaStream_t st);
+                           int use_cool, double courant, double psc, double tsc, double* dt_run, const DtPublish& pub,
+                           cudaStream_t st);
 
 // admesh flags on the device (w2d_mark.cu).  Per slot: lev, the mirror of
 // lp(:,3:4) (sons: first son, son position) and lp(:,5:8) (links), the
