@@ -34,6 +34,7 @@ __global__ void __launch_bounds__(256) k_dt(const int* __restrict__ leaves, int 
 {
   __shared__ double s0[8], s1[8];
   __shared__ bool last;
+  pdl_begin();
   const int nn = n_dev ? *n_dev : n;
   double m0 = 1.e30, m1 = 1e30;
   for (int k = blockIdx.x * blockDim.x + threadIdx.x; k < nn; k += gridDim.x * blockDim.x) {
@@ -84,6 +85,7 @@ __global__ void __launch_bounds__(256) k_dt_runs(const int* __restrict__ leaves,
 {
   __shared__ double s0[8], s1[8];
   const int r = blockIdx.x;
+  pdl_begin();
   double m0 = 1.e30, m1 = 1e30;
   for (int k = loff[r] + threadIdx.x; k < loff[r + 1]; k += blockDim.x) {
     const int b = leaves[k];
@@ -114,8 +116,7 @@ cudaError_t launch_dt_runs(const int* leaves, const int* loff, int nruns, const 
                            cudaStream_t st)
 {
   if (nruns == 0) return cudaSuccess;
-  k_dt_runs<<<nruns, 256, 0, st>>>(leaves, loff, cfl, dtcool, use_cool, courant, psc, tsc, dt_run, pub);
-  return cudaGetLastError();
+  return launch_pdl(k_dt_runs, nruns, 256, 0, st, leaves, loff, cfl, dtcool, use_cool, courant, psc, tsc, dt_run, pub);
 }
 
 __global__ void k_gather_leaf(const int* __restrict__ leaves, int n, const int* __restrict__ n_dev,
@@ -157,8 +158,8 @@ cudaError_t launch_dt(const int* leaves, int n, const int* n_dev, int grid, cons
                       unsigned int* count, double* dt_out, const DtPublish& pub, cudaStream_t st)
 {
   if (grid <= 0) grid = n > 0 ? (n + 255) / 256 : 1;
-  k_dt<<<grid, 256, 0, st>>>(leaves, n, n_dev, cfl, dtcool, use_cool, courant, psc, tsc, work, count, dt_out, pub);
-  return cudaGetLastError();
+  return launch_pdl(k_dt, grid, 256, 0, st, leaves, n, n_dev, cfl, dtcool, use_cool, courant, psc, tsc, work, count,
+                    dt_out, pub);
 }
 
 }  // namespace w2d

@@ -832,6 +832,7 @@ template <typename R, int NEQ, int SOLVER, bool P>
 __global__ void __launch_bounds__(W2D_THREADS, w2d_minb<R>(P)) k_half(KArgs a, PhysArgs pa, double dt)
 {
   bar_init_once(reinterpret_cast<uint64_t*>(w2d_smem));
+  pdl_begin();
   uint32_t par = 0;
   for (LeafRange lr = leaf_range<P>(a); lr.li < lr.end; lr.li += lr.step, par ^= 1u)
     if (!half_leaf<R, NEQ, SOLVER>(a, pa, dt, lr.li, par)) return;
@@ -999,6 +1000,7 @@ template <typename R, int NEQ, int SOLVER, int LIMITER, bool P>
 __global__ void __launch_bounds__(W2D_THREADS, w2d_minb<R>(P)) k_full(KArgs a, PhysArgs pa, double dt)
 {
   bar_init_once(reinterpret_cast<uint64_t*>(w2d_smem));
+  pdl_begin();
   uint32_t par = 0;
   for (LeafRange lr = leaf_range<P>(a); lr.li < lr.end; lr.li += lr.step, par ^= 1u)
     if (!full_leaf<R, NEQ, SOLVER, LIMITER>(a, pa, dt, lr.li, par)) return;
@@ -1064,6 +1066,7 @@ template <typename R, int NEQ, bool P>
 __global__ void __launch_bounds__(256) k_fill1g(KArgs a, PhysArgs pa)
 {
   const int tid = threadIdx.x, g = tid >> 6, t = tid & 63;
+  pdl_begin();
   LeafRange lr;
   if (P) {
     lr = leaf_range<true>(a);
@@ -1105,6 +1108,7 @@ __global__ void __launch_bounds__(W2D_THREADS, w2d_minb<R>(P)) k_calcprim(KArgs 
   const int tid = threadIdx.x;
   const size_t bs = (size_t)NEQ * W2D_CELLS;
   bar_init_once(bar);
+  pdl_begin();
   uint32_t par = 0;
   LeafRange lr = leaf_range<P>(a);
   if (P && list != a.leaves) lr = LeafRange{(int)blockIdx.x, n, (int)gridDim.x};

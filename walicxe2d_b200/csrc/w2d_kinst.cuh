@@ -44,8 +44,7 @@ static cudaError_t half_p(const KArgs& a, const PhysArgs& pa, double dt, cudaStr
   constexpr size_t sm = smem_half<R, NEQ>();
   cudaError_t e = smem_opt_in(k_half<R, NEQ, S, P>, sm, done);
   if (e != cudaSuccess) return e;
-  k_half<R, NEQ, S, P><<<launch_grid(a), W2D_THREADS, sm, st>>>(a, pa, dt);
-  return cudaGetLastError();
+  return launch_pdl(k_half<R, NEQ, S, P>, launch_grid(a), W2D_THREADS, sm, st, a, pa, dt);
 }
 template <int NEQ, int S>
 static cudaError_t half_t(const KArgs& a, const PhysArgs& pa, double dt, cudaStream_t st)
@@ -70,8 +69,7 @@ static cudaError_t full_p(const KArgs& a, const PhysArgs& pa, double dt, cudaStr
   constexpr size_t sm = smem_full<R, NEQ>();
   cudaError_t e = smem_opt_in(k_full<R, NEQ, S, L, P>, sm, done);
   if (e != cudaSuccess) return e;
-  k_full<R, NEQ, S, L, P><<<launch_grid(a), W2D_THREADS, sm, st>>>(a, pa, dt);
-  return cudaGetLastError();
+  return launch_pdl(k_full<R, NEQ, S, L, P>, launch_grid(a), W2D_THREADS, sm, st, a, pa, dt);
 }
 template <int NEQ, int S, int L>
 static cudaError_t full_t(const KArgs& a, const PhysArgs& pa, double dt, cudaStream_t st)
@@ -97,11 +95,8 @@ static cudaError_t full(int neq, const KArgs& a, const PhysArgs& pa, double dt, 
 template <int NEQ>
 static cudaError_t fill1_t(const KArgs& a, const PhysArgs& pa, cudaStream_t st)
 {
-  if (a.grid > 0)
-    k_fill1g<R, NEQ, true><<<a.grid, 256, 0, st>>>(a, pa);
-  else
-    k_fill1g<R, NEQ, false><<<(a.nleaf + 3) / 4, 256, 0, st>>>(a, pa);
-  return cudaGetLastError();
+  if (a.grid > 0) return launch_pdl(k_fill1g<R, NEQ, true>, a.grid, 256, 0, st, a, pa);
+  return launch_pdl(k_fill1g<R, NEQ, false>, (a.nleaf + 3) / 4, 256, 0, st, a, pa);
 }
 
 static cudaError_t fill1(int neq, const KArgs& a, const PhysArgs& pa, cudaStream_t st)
@@ -126,8 +121,7 @@ static cudaError_t calcprim_p(const KArgs& a, const PhysArgs& pa, const int* lis
   constexpr size_t sm = smem_calcprim<R, NEQ>();
   cudaError_t e = smem_opt_in(k_calcprim<R, NEQ, P>, sm, done);
   if (e != cudaSuccess) return e;
-  k_calcprim<R, NEQ, P><<<grid, W2D_THREADS, sm, st>>>(a, pa, list, n, mode);
-  return cudaGetLastError();
+  return launch_pdl(k_calcprim<R, NEQ, P>, grid, W2D_THREADS, sm, st, a, pa, list, n, mode);
 }
 template <int NEQ>
 static cudaError_t calcprim_t(const KArgs& a, const PhysArgs& pa, const int* list, int n, int mode,
@@ -179,8 +173,7 @@ static cudaError_t cool_p(const KArgs& a, const PhysArgs& pa, double dt_s, cudaS
   constexpr size_t sm = smem_cool<R, NEQ>();
   cudaError_t e = smem_opt_in(k_cool<R, NEQ, P>, sm, done);
   if (e != cudaSuccess) return e;
-  k_cool<R, NEQ, P><<<launch_grid(a), W2D_COOL_THREADS, sm, st>>>(a, pa, dt_s);
-  return cudaGetLastError();
+  return launch_pdl(k_cool<R, NEQ, P>, launch_grid(a), W2D_COOL_THREADS, sm, st, a, pa, dt_s);
 }
 template <int NEQ>
 static cudaError_t cool_t(const KArgs& a, const PhysArgs& pa, double dt_s, cudaStream_t st)

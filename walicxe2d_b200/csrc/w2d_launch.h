@@ -8,6 +8,28 @@
 
 namespace w2d {
 
+// Launch of a kernel that calls pdl_begin: it may start while its predecessor
+// on the stream flushes (in a captured graph: a programmatic edge).  64x64
+// mesh, 20 steps with state in and out: 694 us with ordinary launches, 705
+// with the successor let in from the predecessor's start, 660 so; cylindrical
+// jet (no graphs), 16 steps: 1,925 / 1,840 / 1,756 us; 8,835 blocks, 20 steps:
+// 11.12 / 11.27 / 11.03 ms.
+template <class... P, class... A>
+cudaError_t launch_pdl(void (*kernel)(P...), int grid, int block, size_t smem, cudaStream_t st, A... args)
+{
+  cudaLaunchConfig_t cfg = {};
+  cfg.gridDim = dim3((unsigned)grid);
+  cfg.blockDim = dim3((unsigned)block);
+  cfg.dynamicSmemBytes = smem;
+  cfg.stream = st;
+  cudaLaunchAttribute attr[1];
+  attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+  attr[0].val.programmaticStreamSerializationAllowed = 1;
+  cfg.attrs = attr;
+  cfg.numAttrs = 1;
+  return cudaLaunchKernelEx(&cfg, kernel, static_cast<P>(args)...);
+}
+
 struct Launchers {
   cudaError_t (*half)(int neq, const KArgs&, const PhysArgs&, double dt, cudaStream_t);
   cudaError_t (*full)(int neq, const KArgs&, const PhysArgs&, double dt, cudaStream_t);

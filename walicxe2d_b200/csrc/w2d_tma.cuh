@@ -64,4 +64,14 @@ __device__ __forceinline__ bool mbar_wait(uint64_t* bar, uint32_t parity)
   return false;
 }
 
+// Programmatic dependent launch.  The step's kernels are launched so that
+// each may start once its predecessor's CTAs have left (launch_pdl), without
+// waiting for the flush and the launch behind it; every one of them calls
+// pdl_begin before it reads anything another kernel wrote, which waits until
+// the predecessors have completed and their writes are visible.  No kernel
+// lets its successor in earlier (griddepcontrol.launch_dependents at the start
+// measured slower: CTAs waiting beside the predecessor's last ones).  In a
+// kernel launched the ordinary way it is a no-op.
+__device__ __forceinline__ void pdl_begin() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
+
 }  // namespace w2d
