@@ -142,6 +142,15 @@ int launch_tk(W2dCtx* c, int tk, const char* name, F fn)
   return rc;
 }
 
+// the captured sequences of the separate kernels' steps
+void drop_step_graphs(W2dCtx* c)
+{
+  if (c->gx_first) cudaGraphExecDestroy(c->gx_first);
+  if (c->gx_rest) cudaGraphExecDestroy(c->gx_rest);
+  if (c->gx_whole) cudaGraphExecDestroy(c->gx_whole);
+  c->gx_first = c->gx_rest = c->gx_whole = nullptr;
+}
+
 // After a synchronization: the tuned kernels' times of the last step go to
 // the shape in use; after the last tuning step every kernel keeps its
 // fastest shape and the step graphs are captured anew.
@@ -175,9 +184,7 @@ void tune_collect(W2dCtx* c)
       }
     c->tshape[k] = best;
   }
-  if (c->gx_first) cudaGraphExecDestroy(c->gx_first);
-  if (c->gx_rest) cudaGraphExecDestroy(c->gx_rest);
-  c->gx_first = c->gx_rest = nullptr;
+  drop_step_graphs(c);
 }
 
 KArgs kargs(W2dCtx* c, const int2* fd)
@@ -521,6 +528,11 @@ int half_step(W2dCtx* c, double dt, const double* dt_dev)
 // ---------------------------------------------------------------------------
 // the split timestep/tstep of w2d_internal.h
 
+static DtPublish dt_publish(W2dCtx* c, double* dt_host)
+{
+  return {dt_host, c->h_err, c->d_err, c->d_queue, c->h_hist, c->hist_cap, std::max(c->nruns, 1), c->d_nleaf};
+}
+
 // src/timestep.f90:7-61 as one reduction kernel; dt stays in device memory,
 // and the kernel stores it, with the error word, to pinned memory where pub
 // says so
@@ -556,7 +568,7 @@ int ctx_dt_publish(W2dCtx* c)
 
 int ctx_dt_launch(W2dCtx* c)
 {
-  int rc = dt_reduce(c, DtPublish{c->h_small, c->h_err, c->d_err});
+  int rc = dt_reduce(c, dt_publish(c, c->h_small));
   if (rc) return rc;
   if (!c->capturing) CK(cudaEventRecord(c->ev_dt, c->st));
   return W2D_OK;
@@ -813,8 +825,7 @@ int w2d_destroy(W2dCtx* c)
   cudaEvent_t evs[] = {c->ev_topo, c->ev_ops, c->ev_plan[0], c->ev_plan[1], c->ev_dt, c->ev_links};
   for (auto e : evs)
     if (e) cudaEventDestroy(e);
-  if (c->gx_first) cudaGraphExecDestroy(c->gx_first);
-  if (c->gx_rest) cudaGraphExecDestroy(c->gx_rest);
+  drop_step_graphs(c);
   if (c->gx_step) cudaGraphExecDestroy(c->gx_step);
   for (int k = 0; k < 5; ++k)
     for (int q = 0; q < 2; ++q)
@@ -823,10 +834,12 @@ int w2d_destroy(W2dCtx* c)
   void* dev2[] = {c->d_run_of, c->d_runs, c->d_dt_run, c->d_loff, c->d_gradleaf, c->d_fb, c->d_fb_count,
                   c->d_nn_counts, c->d_nleaf, c->d_links, c->d_sons, c->d_mflags, c->d_mlists, c->d_rows7,
                   c->d_posof, c->d_bent, c->d_bspan, c->d_blocal, c->d_bcta, c->d_wpos,
-                  c->d_step_flags, c->d_step_sync, c->d_step_part};
+                  c->d_step_flags, c->d_step_sync, c->d_step_part, c->d_queue};
   for (void* d : dev2)
     if (d) cudaFree(d);
   if (c->h_dt_run) cudaFreeHost(c->h_dt_run);
+  if (c->h_queue) cudaFreeHost(c->h_queue);
+  if (c->h_hist) cudaFreeHost(c->h_hist);
   if (c->h_mlists) cudaFreeHost(c->h_mlists);
   if (c->h_rows7) cudaFreeHost(c->h_rows7);
   if (c->h_loff) cudaFreeHost(c->h_loff);
@@ -1779,7 +1792,7 @@ int ctx_ens_dt_launch(W2dCtx* c)
   int rc = launch(c, "timestep", [&] {
     return launch_dt_runs(c->d_leaves, c->d_loff, c->nruns, c->d_cfl, c->d_dtcool,
                           c->p.cooling == W2D_COOLINGDMC, c->p.cfl, c->p.psc, c->p.tsc, c->d_dt_run,
-                          DtPublish{c->h_dt_run, c->h_err, c->d_err}, c->st);
+                          dt_publish(c, c->h_dt_run), c->st);
   });
   return rc;
 }
@@ -2039,6 +2052,83 @@ int ctx_step_rest(W2dCtx* c)
   return W2D_OK;
 }
 
+// Steps queued without a wait between them: runs whose mesh stays (no
+// admesh) and whose dt stays on the device.  Each step is then one graph of
+// the two sequences above (or their launches); the host waits once per batch
+// and takes the steps' dt from the history the reduction kept.
+constexpr int kQueueSteps = 128;
+
+int ctx_queue_max(W2dCtx* c)
+{
+  const bool dev_dt = c->nruns > 0 || ctx_device_dt(c);
+  if (!dev_dt || c->tune_left > 0 || c->prof || step_fused_ok(c) || !c->have_topology || !c->have_bounds ||
+      c->leaves_dirty)
+    return 0;
+  return kQueueSteps;
+}
+
+static int queue_steps(W2dCtx* c, int n)
+{
+  int rc;
+  auto body = [&] {
+    int r = c->nruns > 0 ? ctx_ens_dt_launch(c) : ctx_dt_launch(c);
+    if (!r) r = ctx_half_step(c);
+    return r ? r : ctx_tstep_rest(c, 0.0, 0.0);
+  };
+  if (!graphs_now(c)) {
+    for (int k = 0; k < n; ++k)
+      if ((rc = body())) return rc;
+    return W2D_OK;
+  }
+  if (c->nn_img) {
+    bool moved = false;
+    if ((rc = ensure_fb(c, &moved))) return rc;
+    if (moved) drop_step_graphs(c);
+  }
+  if (!c->gx_whole && (rc = capture(c, &c->gx_whole, &c->nlaunch_graph_whole, body))) return rc;
+  for (int k = 0; k < n; ++k) {
+    CK(cudaGraphLaunch(c->gx_whole, c->st));
+    c->nlaunch += c->nlaunch_graph_whole;
+  }
+  return W2D_OK;
+}
+
+int ctx_queue_run(W2dCtx* c, int n, int* done, const double** dts)
+{
+  *done = 0;
+  *dts = c->h_hist;
+  const int runs = std::max(c->nruns, 1);
+  int rc;
+  if (!c->d_queue) {
+    // (allocated once; graphs captured before hold a reduction without it)
+    CK(cudaStreamSynchronize(c->st));
+    drop_step_graphs(c);
+    CK(cudaMalloc(&c->d_queue, sizeof(int) * (size_t)(2 + runs)));
+    CK(cudaMemsetAsync(c->d_queue, 0, sizeof(int) * (size_t)(2 + runs), c->st));
+    CK(cudaMallocHost(&c->h_queue, sizeof(int) * (size_t)(2 + runs)));
+    CK(cudaMallocHost(&c->h_hist, sizeof(double) * (size_t)kQueueSteps * runs));
+    c->hist_cap = kQueueSteps;
+    *dts = c->h_hist;
+  }
+  n = std::min(n, c->hist_cap);
+  memset(c->h_queue, 0, sizeof(int) * (size_t)(2 + runs));
+  c->h_queue[1] = 1;
+  CK(cudaMemcpyAsync(c->d_queue, c->h_queue, sizeof(int) * (size_t)(2 + runs), cudaMemcpyHostToDevice, c->st));
+  rc = queue_steps(c, n);
+  if (!rc) {
+    CK(cudaMemcpyAsync(c->h_queue, c->d_queue, sizeof(int) * (size_t)(2 + runs), cudaMemcpyDeviceToHost, c->st));
+    rc = sync_and_check(c);
+    *done = c->h_queue[2];
+  }
+  CK(cudaMemsetAsync(c->d_queue, 0, 2 * sizeof(int), c->st));
+  if (rc) {   // the count the reduction set to 0 behind the failed step
+    c->h_nleaf[0] = c->nleaf;
+    CK(cudaMemcpyAsync(c->d_nleaf, c->h_nleaf, sizeof(int), cudaMemcpyHostToDevice, c->st));
+    CK(cudaStreamSynchronize(c->st));
+  }
+  return rc;
+}
+
 extern "C" {
 
 int w2d_autotune(W2dCtx* c, int reps)
@@ -2070,10 +2160,9 @@ int w2d_set_graphs(W2dCtx* c, int on)
   if (c->want_graphs)   // a captured launch needs a grid independent of the leaf count
     for (int k = 0; k < TK_N; ++k)
       if (kShapes[c->tshape[k]].per_sm == 0) c->tshape[k] = 2;
-  if (c->gx_first) cudaGraphExecDestroy(c->gx_first);
-  if (c->gx_rest) cudaGraphExecDestroy(c->gx_rest);
+  drop_step_graphs(c);
   if (c->gx_step) cudaGraphExecDestroy(c->gx_step);
-  c->gx_first = c->gx_rest = c->gx_step = nullptr;
+  c->gx_step = nullptr;
   return W2D_OK;
 }
 

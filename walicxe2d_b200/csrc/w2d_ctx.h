@@ -78,6 +78,14 @@ struct W2dCtx {
   bool dt_on_device = false;
   cudaGraphExec_t gx_first = nullptr, gx_rest = nullptr;
   int64_t nlaunch_graph_first = 0, nlaunch_graph_rest = 0;
+  // steps queued without a wait (ctx_queue_*): the counters the time-step
+  // reduction keeps, the dt of every queued step, the graph of a whole step
+  int* d_queue = nullptr;       // [2 + runs] (DtPublish)
+  double* h_hist = nullptr;     // pinned [hist_cap][runs]
+  int* h_queue = nullptr;       // pinned [2 + runs]
+  int hist_cap = 0;
+  cudaGraphExec_t gx_whole = nullptr;
+  int64_t nlaunch_graph_whole = 0;
   // the fused step kernel (w2d_step.cuh), allocated by its first use: per
   // slot the epochs of the last half and full step, the epoch and barrier
   // words, the CTAs' CFL minima; its grid (-1: not sized yet, 0: it does

@@ -323,6 +323,29 @@ int w2d_ens_run(W2dEns* e, int nsteps)
     const double t0 = now_ms();
     bool any = false;
     for (int r = 0; r < nr; ++r) any = any || e->dirty[r];
+    // meshes that stay: as many steps as may be queued at once, one wait
+    const int m = e->amr || any ? 0 : std::min(nsteps - n, ctx_queue_max(e->ctx));
+    if (m > 1) {
+      int done = 0;
+      const double* dts = nullptr;
+      rc = ctx_queue_run(e->ctx, m, &done, &dts);
+      for (auto& s : e->runs) s.zone_updates += (int64_t)done * s.nbleafs * s.p.nx * s.p.ny;
+      for (int k = 0; k < (rc ? done - 1 : done); ++k) {
+        for (int r = 0; r < nr; ++r) {
+          W2dSim& s = e->runs[r];
+          s.dt = dts[(size_t)k * nr + r];
+          s.time = s.time + s.dt;                                 // src/main.f90:88
+          s.steps++;
+        }
+        e->steps++;
+      }
+      const double ms = now_ms() - t0;
+      e->phase_ms[1] += ms;
+      e->phase_ms[7] += ms;
+      if (rc) return rc;
+      n += m - 1;
+      continue;
+    }
     if (any && (rc = push_leaves(e))) return rc;
     const double t1 = now_ms();
     if ((rc = ctx_step_first(e->ctx))) return rc;    // src/main.f90:87 for every run, then tstep's first pass

@@ -663,6 +663,28 @@ int w2d_sim_run(W2dSim* s, int nsteps)
   // before the full step
   const bool dev_dt = ctx_device_dt(s->ctx);
   for (int n = 0; n < nsteps && dev_dt; ++n) {
+    // a mesh that stays: as many steps as may be queued at once, one wait
+    if (!s->amr && !s->dirty) {
+      const int m = std::min(nsteps - n, ctx_queue_max(s->ctx));
+      if (m > 1) {
+        const double t0 = now_ms();
+        int done = 0;
+        const double* dts = nullptr;
+        rc = ctx_queue_run(s->ctx, m, &done, &dts);
+        s->zone_updates += (int64_t)done * s->nbleafs * s->p.nx * s->p.ny;
+        for (int k = 0; k < (rc ? done - 1 : done); ++k) {
+          s->dt = dts[k];
+          s->time = s->time + s->dt;                           // src/main.f90:88
+          s->steps++;
+        }
+        const double ms = now_ms() - t0;
+        s->phase_ms[1] += ms;
+        s->phase_ms[8] += ms;
+        if (rc) return rc;
+        n += m - 1;
+        continue;
+      }
+    }
     // step graphs: dt stays on the device (the kernels read it there) and
     // comes to the host with the step's synchronization
     tree_trial_pre(s);

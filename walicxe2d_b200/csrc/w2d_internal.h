@@ -119,6 +119,13 @@ int ctx_ens_criteria(W2dCtx* c, const double** grad);
 // w2d_set_graphs, captured again after tuning or when a buffer moves)
 int ctx_step_first(W2dCtx* c);
 int ctx_step_rest(W2dCtx* c);
+// Steps without a wait between them, for a mesh that stays: ctx_queue_max is
+// how many may be queued at once (0: not now), ctx_queue_run queues n and
+// waits for them.  *done: steps begun without an error, (*dts)[k * runs + r]
+// the dt of run r in the k-th.  After an error the last of them is the step
+// that failed; the steps queued behind it left the state alone.
+int ctx_queue_max(W2dCtx* c);
+int ctx_queue_run(W2dCtx* c, int n, int* done, const double** dts);
 // a single run steps through ctx_step_first/rest (w2d_set_graphs on, no jet)
 bool ctx_device_dt(W2dCtx* c);
 // the dt copied by the last ctx_dt_launch (valid after a synchronization)
