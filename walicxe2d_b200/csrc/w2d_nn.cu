@@ -114,6 +114,99 @@ __global__ void k_nn_samples_dmc(int64_t n, uint64_t seed, const double* __restr
   targ[ld + k] = t[1];
 }
 
+// The exact routine as the training labels and the judge take it: atomic
+// (src/coolingh.f90:171-254) with CUDA's own calls, one at a time.  It runs
+// once per sample, so it is not bound by their cost as the cooling kernel is,
+// whose form of the same routine (d_atomic_core) rounds differently in the last
+// place; a label is a difference y1 - y0 taken to its logarithm, which carries
+// that last place into the weights, and training here repeats the networks
+// trained before.
+// alpha (src/coolingh.f90: 2.55e-13 (1e4/T)**0.79), from lT = log(T)
+__device__ __forceinline__ double nn_label_alpha(double lT) { return 2.55e-13 * exp(0.79 * (kLn1e4 - lT)); }
+__device__ __forceinline__ double nn_label_colf(double T) { return 5.83e-11 * sqrt(T) * exp(-157828. / T); }
+// betah: a = 157890/T, 1.133e-24/sqrt(a) (-0.0713 + 0.5 log a + 0.640 a**(-0.33333))
+__device__ __forceinline__ double nn_label_betah(double T, double lT)
+{
+  const double a = 157890. / T;
+  const double la = kLn157890 - lT;
+  return 1.133e-24 / sqrt(a) * (-0.0713 + 0.5 * la + 0.640 * exp(-0.33333 * la));
+}
+
+// src/coolingh.f90:88-165 (ALOSS), with lte0 = log(te0)
+__device__ __forceinline__ double nn_label_aloss(double x1, double den, double dh0, double te0, double lte0)
+{
+  const double XO = 1.e-3, XION = 2.179e-11;
+  const double C0 = 0.5732, C1 = 1.8288e-5, C2 = -1.15822e-10, C3 = 9.4288e-16;
+  const double D0 = 0.5856, D1 = 1.55083e-5, D2 = -9.669e-12, D3 = 5.716e-19;
+  const double ENK = 118409., EN = 1.634E-11;
+  double te = fmaxr(te0, 1000.);
+  const double lte = te0 > 1000. ? lte0 : kLn1e3;
+  double dh = den;
+  double dhp = (1. - x1) * dh;
+  double de = dhp + 1.E-4 * dh;
+  double doi = XO * dh0;
+  double doii = XO * dhp;
+  double omega = 0.;
+  if (te <= 55000.) omega = C0 + te * (C1 + te * (C2 + te * C3));
+  if (te >= 72000.) omega = D0 + te * (D1 + te * (D2 + te * D3));
+  if (te > 55000. && te < 72000.) {
+    double omegal = C0 + te * (C1 + te * (C2 + te * C3));
+    double omegah = D0 + te * (D1 + te * (D2 + te * D3));
+    double frac = (te - 55000.) / 17000.;
+    omega = (1. - frac) * omegal + frac * omegah;
+  }
+  double qla = 8.6287E-6 / (2. * sqrt(te)) * omega * exp(-ENK / te);
+  double ecoll = fmaxr(de * dh0 * qla * EN, 0.);
+  double cion = 5.834E-11 * sqrt(te) * exp(-1.579E5 / te);
+  double eion = de * dh0 * cion * XION;
+  double erec = fmaxr(de * dhp * (nn_label_betah(te, lte)), 0.);
+  double tm = 1. / te;
+  double t2 = tm * tm;
+  double eoi = fmaxr(de * doi * exp10(1381465. * t2 - 12328.69 * tm - 19.82621), 0.);
+  double eoii = fmaxr(de * doii * exp10(-2061075. * t2 - 14596.24 * tm - 19.01402), 0.);
+  double betaf = 1.3 * 1.42E-27 * sqrt(te);
+  double hiicool = de * dhp * betaf;
+  double equil = (1.0455E-18 / exp(0.63 * lte)) * (1. - exp(-exp(1.63 * (lte - kLn1e5)))) * de * den + hiicool;
+  double fr = 0.;
+  if (te >= 54770.) fr = 1.;
+  if (te > 44770. && te < 54770.) {
+    double ex2 = exp(-2. * (te - 49770.) / 500.);
+    double th = (1. - ex2) / (1. + ex2);
+    fr = 0.5 * (1. + th);
+  }
+  return ecoll + eion + (erec + 7.033 * (eoi + eoii)) * (1. - fr) + equil * fr;
+}
+
+// src/coolingh.f90:171-254 (atomic) in FP64 on one cell: from the
+// temperature T, neutral fraction y0, density dh and dt (s), the new
+// neutral fraction y1, the cooling rate ce of the temperature relaxation
+// t1 = 10 + (T - 10) exp(-ce dt) and the clamped new temperature t1.
+__device__ __forceinline__ void nn_label_atomic(double T, double y0, double dh, double dt, double& y1, double& ce,
+                                              double& t1)
+{
+  const double xi = 1.e-4, boltzm = 1.3807e-16;
+  const double lT = log(T);
+  double col = nn_label_colf(T);
+  double rec = nn_label_alpha(lT);
+  double a = rec + col;
+  double b = -((2. + xi) * rec + (1. + xi) * col);
+  double c = (1. + xi) * rec;
+  double d = sqrt(b * b - 4. * a * c);
+  double g0 = (2. * a * y0 + b + d) / (2. * a * y0 + b - d);
+  double e = exp(-d * dh * dt);
+  y1 = (-b - d * (1. + g0 * e) / (1. - g0 * e)) / (2. * a);
+  y1 = fminr(y1, 1.);
+  y1 = fmaxr(y1, 0.0001);
+  double dh0 = y1 * dh;
+  double al = nn_label_aloss(y0, dh, dh0, T, lT) / (dh * dh);
+  double tprime = 10.;
+  ce = (2. * dh * al) / (3. * boltzm * T);
+  t1 = tprime + (T - tprime) * exp(-ce * dt);
+  t1 = fmaxr(t1, 0.1 * T);
+  t1 = fminr(t1, 10. * T);
+  t1 = fmaxr(t1, tprime);
+}
+
 // Training set labelled by the exact routine (atomic, src/coolingh.f90).
 __global__ void k_nn_samples(int64_t n, uint64_t seed, int64_t i0, float* __restrict__ feat,
                              float* __restrict__ targ, int64_t ld)
@@ -122,7 +215,7 @@ __global__ void k_nn_samples(int64_t n, uint64_t seed, int64_t i0, float* __rest
   if (k >= n) return;
   double dn, T, y0, dts, y1, ce, t1;
   nn_draw(seed, i0 + k, dn, T, y0, dts);
-  d_atomic_core(T, y0, dn, dts, y1, ce, t1);
+  nn_label_atomic(T, y0, dn, dts, y1, ce, t1);
   float f[4], t[2];
   nn_features(dn, T, y0, dts, f);
   nn_targets(dn, y0, dts, y1, ce, t);
@@ -509,7 +602,7 @@ __global__ void k_nn_judge(int64_t n, uint64_t seed, const float* __restrict__ o
     return;
   }
   double y1, ce, t1, y1p, t1p;
-  d_atomic_core(T, y0, dn, dts, y1, ce, t1);
+  nn_label_atomic(T, y0, dn, dts, y1, ce, t1);
   const bool use = nn_update(out[k], out[n + k], dn, T, y0, dts, y1p, t1p, tol);
   res[k] = use ? 1.f : 0.f;
   res[n + k] = (float)fabs(t1p / t1 - 1.);
