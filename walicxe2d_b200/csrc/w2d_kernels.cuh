@@ -554,8 +554,7 @@ __device__ __forceinline__ void block_stats(const R (*sp)[W2D_W][W2D_W], const P
   const int i = 1 + tid % 16, j = 1 + tid / 16;
   const int ti = i + 1, tj = j + 1;
   const R rho = sp[0][tj][ti], vx = sp[1][tj][ti], vy = sp[2][tj][ti], p = sp[3][tj][ti];
-  const typename DenOf<R>::T dn = den(rho);
-  const R cs = sound(ph, p, dn);
+  const R cs = sound(ph, p, rho);
   const R au = warp_max0(absr(vx) + cs), av = warp_max0(absr(vy) + cs);
   const R am = fmaxr(R(1e-15), absr(p));   // (rho, above the same floor, is its own scale)
   R dp = absr(sp[3][tj][ti + 1] - p);
@@ -566,7 +565,7 @@ __device__ __forceinline__ void block_stats(const R (*sp)[W2D_W][W2D_W], const P
   dr = fmaxr(dr, absr(sp[0][tj][ti - 1] - rho));
   dr = fmaxr(dr, absr(sp[0][tj + 1][ti] - rho));
   dr = fmaxr(dr, absr(sp[0][tj - 1][ti] - rho));
-  const R grad = warp_max0(fmaxr(divr(dp, am), quot(dr, dn)));
+  const R grad = warp_max0(fmaxr(divr(dp, am), divr(dr, rho)));
   double dtc = 1e30;
   if (pa.cooling == COOL_DMC) {                    // src/timestep.f90:34-41
     const double T = ((double)p / (double)rho) * pa.tempsc;
@@ -635,13 +634,12 @@ __device__ __forceinline__ void interior_stats(R (*st)[W2D_W][W2D_W], double* sr
   const int i = 1 + tid % 16, j = 1 + tid / 16;
   const int ti = i + 1, tj = j + 1;
   R au = R(0.), av = R(0.), rho = R(0.), p = R(0.);
-  typename DenOf<R>::T dn;
   if (tid < 256) {
     R q[NEQ], nv[NEQ], T;
 #pragma unroll
     for (int k = 0; k < NEQ; ++k) nv[k] = st[k][tj][ti];
-    uprim<NEQ>(ph, q, nv, T, dn);
-    const R cs = sound(ph, q[3], dn);
+    uprim<NEQ>(ph, q, nv, T);
+    const R cs = sound(ph, q[3], q[0]);
     au = absr(q[1]) + cs;
     av = absr(q[2]) + cs;
     rho = q[0];
@@ -660,7 +658,7 @@ __device__ __forceinline__ void interior_stats(R (*st)[W2D_W][W2D_W], double* sr
     if (i > 1) { dp = fmaxr(dp, absr(st[3][tj][ti - 1] - p)); dr = fmaxr(dr, absr(st[0][tj][ti - 1] - rho)); }
     if (j < W2D_NX) { dp = fmaxr(dp, absr(st[3][tj + 1][ti] - p)); dr = fmaxr(dr, absr(st[0][tj + 1][ti] - rho)); }
     if (j > 1) { dp = fmaxr(dp, absr(st[3][tj - 1][ti] - p)); dr = fmaxr(dr, absr(st[0][tj - 1][ti] - rho)); }
-    const R grad = warp_max0(fmaxr(divr(dp, am), quot(dr, dn)));
+    const R grad = warp_max0(fmaxr(divr(dp, am), divr(dr, rho)));
     au = warp_max0(au);
     av = warp_max0(av);
     if ((tid & 31) == 0) {
@@ -702,15 +700,8 @@ __device__ __forceinline__ double cyl_radius(const KArgs& a, int b, int lev, int
 template <typename R, int NEQ>
 __host__ __device__ constexpr size_t smem_half()
 {
-  return 128 + sizeof(R) * ((2 * NEQ + 1 + (sizeof(R) == 4)) * W2D_CELLS + 2 * NEQ * 272);
+  return 128 + sizeof(R) * (2 * NEQ * W2D_CELLS + W2D_CELLS + 2 * NEQ * 272);
 }
-
-// the density rho as a divisor, its reciprocal read back in FP32
-__device__ __forceinline__ Den64 kept_den(double rho, const double*) { return {rho}; }
-__device__ __forceinline__ Den32 kept_den(float, const float* y) { return {*y}; }
-// one of two densities as a divisor (rho: the one chosen)
-__device__ __forceinline__ Den64 either(const Den64&, const Den64&, bool, double rho) { return {rho}; }
-__device__ __forceinline__ Den32 either(const Den32& l, const Den32& r, bool left, float) { return {left ? l.y : r.y}; }
 
 // One leaf of the half step (position li of the leaf list); the tile
 // barrier completes with phase parity `par`.  Returns false when the tile
@@ -719,17 +710,13 @@ template <typename R, int NEQ, int SOLVER, bool U = false>
 __device__ __forceinline__ bool half_leaf(const KArgs& a, const PhysArgs& pa, double dt, int li, uint32_t par)
 {
   // su: the tile as loaded (u, or the stored primitives under DMC); st:
-  // the primitives of cells 0..17; scs: their sound speeds; siv
-  // (FP32): the reciprocals of their densities
+  // the primitives of cells 0..17; scs: their sound speeds
   uint64_t* bar = reinterpret_cast<uint64_t*>(w2d_smem);
   R(*su)[W2D_W][W2D_W] = reinterpret_cast<R(*)[W2D_W][W2D_W]>(w2d_smem + 128);
   R(*st)[W2D_W][W2D_W] = reinterpret_cast<R(*)[W2D_W][W2D_W]>(w2d_smem + 128 + sizeof(R) * NEQ * W2D_CELLS);
   R(*scs)[W2D_W] = reinterpret_cast<R(*)[W2D_W]>(w2d_smem + 128 + sizeof(R) * 2 * NEQ * W2D_CELLS);
-  R(*siv)[W2D_W] = reinterpret_cast<R(*)[W2D_W]>(w2d_smem + 128 + sizeof(R) * (2 * NEQ + 1) * W2D_CELLS);
-  constexpr bool inv = sizeof(R) == 4;
-  constexpr int NT = 2 * NEQ + 1 + inv;   // tiles
-  R(*sf)[16][17] = reinterpret_cast<R(*)[16][17]>(w2d_smem + 128 + sizeof(R) * NT * W2D_CELLS);
-  R(*sg)[17][16] = reinterpret_cast<R(*)[17][16]>(w2d_smem + 128 + sizeof(R) * (NT * W2D_CELLS + NEQ * 272));
+  R(*sf)[16][17] = reinterpret_cast<R(*)[16][17]>(w2d_smem + 128 + sizeof(R) * (2 * NEQ + 1) * W2D_CELLS);
+  R(*sg)[17][16] = reinterpret_cast<R(*)[17][16]>(w2d_smem + 128 + sizeof(R) * ((2 * NEQ + 1) * W2D_CELLS + NEQ * 272));
   const Phys<R> ph = make_phys<R, SOLVER, -1>(pa);
   const int tid = threadIdx.x;
   const size_t bs = (size_t)NEQ * W2D_CELLS;
@@ -760,19 +747,15 @@ __device__ __forceinline__ bool half_leaf(const KArgs& a, const PhysArgs& pa, do
     R q[NEQ];
 #pragma unroll
     for (int k = 0; k < NEQ; ++k) q[k] = su[k][tj][ti];
-    typename DenOf<R>::T dn;
     if (!dmc) {
       R uu[NEQ], T;
 #pragma unroll
       for (int k = 0; k < NEQ; ++k) uu[k] = q[k];
-      uprim<NEQ>(ph, q, uu, T, dn);
-    } else {
-      dn = den(q[0]);
+      uprim<NEQ>(ph, q, uu, T);
     }
 #pragma unroll
     for (int k = 0; k < NEQ; ++k) st[k][tj][ti] = q[k];
-    scs[tj][ti] = sound(ph, q[3], dn);
-    if constexpr (inv) siv[tj][ti] = dn.y;
+    scs[tj][ti] = sound(ph, q[3], q[0]);
   }
   __syncthreads();
 
@@ -797,8 +780,7 @@ __device__ __forceinline__ bool half_leaf(const KArgs& a, const PhysArgs& pa, do
       pr[0] = t[n]; pr[1] = t[p1 + n]; pr[2] = t[p2 + n];
 #pragma unroll
       for (int k = 3; k < NEQ; ++k) { pl[k] = t[k * W2D_CELLS + c]; pr[k] = t[k * W2D_CELLS + n]; }
-      if (!riemann<NEQ>(ph, pl, pr, cs[c], cs[n],
-                        [&](bool left, R rho) { return kept_den(rho, &siv[0][0] + (left ? c : n)); }, ff))
+      if (!riemann<NEQ>(ph, pl, pr, cs[c], cs[n], ff))
         set_err(a.err, ERR_HLLC, b, i, j);
       R* f = (dir ? &sg[0][0][0] : &sf[0][0][0]) + tid;
       f[0] = ff[0];
@@ -952,9 +934,8 @@ __device__ __forceinline__ bool full_leaf(const KArgs& a, const PhysArgs& pa, do
         pr[k] = q[s];
         limit1<R>(ph.limiter, q[-s], pl[k], pr[k], q[2 * s]);
       }
-      const typename DenOf<R>::T dl = den(pl[0]), dr = den(pr[0]);
-      const R csl = sound(ph, pl[3], dl), csr = sound(ph, pr[3], dr);
-      if (!riemann<NEQ>(ph, pl, pr, csl, csr, [&](bool left, R rho) { return either(dl, dr, left, rho); }, ff))
+      const R csl = sound(ph, pl[3], pl[0]), csr = sound(ph, pr[3], pr[0]);
+      if (!riemann<NEQ>(ph, pl, pr, csl, csr, ff))
         set_err(a.err, ERR_HLLC, b, i, j);
       R* f = (dir ? &sg[0][0][0] : &sf[0][0][0]) + tid;
       f[0] = ff[0];

@@ -34,8 +34,13 @@ __device__ __forceinline__ float signr(float a) { return copysignf(1.0f, a); }
 // y + x/2 and y - x/2 (halving is exact, so one operation rounds as two)
 __device__ __forceinline__ double add_half(double y, double x) { return fma(0.5, x, y); }
 __device__ __forceinline__ double sub_half(double y, double x) { return fma(-0.5, x, y); }
-__device__ __forceinline__ float add_half(float y, float x) { return y + 0.5f * x; }
-__device__ __forceinline__ float sub_half(float y, float x) { return y - 0.5f * x; }
+__device__ __forceinline__ float add_half(float y, float x) { return y + x * 0.5f; }
+__device__ __forceinline__ float sub_half(float y, float x) { return y - x * 0.5f; }
+// r v2 / 2 + y and y - r v2 / 2 (FP32 contracts its products by itself)
+__device__ __forceinline__ double kin_plus(double r, double v2, double y) { return fma(0.5, r * v2, y); }
+__device__ __forceinline__ double minus_kin(double y, double r, double v2) { return fma(-0.5, r * v2, y); }
+__device__ __forceinline__ float kin_plus(float r, float v2, float y) { return 0.5f * r * v2 + y; }
+__device__ __forceinline__ float minus_kin(float y, float r, float v2) { return y - 0.5f * r * v2; }
 
 enum { SOLVER_HLLC = 0, SOLVER_HLL = 1, SOLVER_HLL_HLLC = 2 };
 enum { COOL_NONE = 0, COOL_H = 1, COOL_DMC = 2 };
@@ -84,58 +89,30 @@ __device__ __forceinline__ double div_cv(const Phys<double>& ph, double x)
 }
 __device__ __forceinline__ float div_cv(const Phys<float>& ph, float x) { return x / ph.cv; }
 
-// A divisor that several quotients share (a cell's velocities and sound speed,
-// an interface's sound speed and star energy all divide by the density).  In
-// FP32 its reciprocal is formed once and each quotient is a product (as near
-// to the quotient as the build's approximate division).  In FP64 every
-// quotient stays the correctly rounded division: a reciprocal with two
-// exact-remainder corrections per quotient rounds the same but measured 6%
-// slower in the full step (198 -> 211 us on 8,835 blocks).
-struct Den64 {
-  double b;
-};
-struct Den32 {
-  float y;
-};
-template <typename R> struct DenOf { using T = Den64; };
-template <> struct DenOf<float> { using T = Den32; };
-__device__ __forceinline__ Den64 den(double b) { return {b}; }
-__device__ __forceinline__ Den32 den(float b) { return {1.f / b}; }
-__device__ __forceinline__ double quot(double a, const Den64& d) { return a / d.b; }
-__device__ __forceinline__ float quot(float a, const Den32& d) { return a * d.y; }
-
 // src/uprim.f90:5-63 -- prim from u; T is returned for the cooling modes.
-// dn: the density (prim[0]) as a divisor, for the caller's own quotients.
 template <int NEQ, typename R>
-__device__ __forceinline__ void uprim(const Phys<R>& ph, R* prim, const R* uu, R& T, typename DenOf<R>::T& dn)
+__device__ __forceinline__ void uprim(const Phys<R>& ph, R* prim, const R* uu, R& T)
 {
   const R tiny = R(1e-15);
   R r = uu[0] > tiny ? uu[0] : tiny;
-  dn = den(r);
   prim[0] = r;
-  prim[1] = quot(uu[1], dn);
-  prim[2] = quot(uu[2], dn);
+  prim[1] = divr(uu[1], r);
+  prim[2] = divr(uu[2], r);
 #pragma unroll
   for (int k = 4; k < NEQ; ++k) prim[k] = uu[k];
-  prim[3] = div_cv(ph, sub_half(uu[3], r * (prim[1] * prim[1] + prim[2] * prim[2])));
+  prim[3] = div_cv(ph, minus_kin(uu[3], r, prim[1] * prim[1] + prim[2] * prim[2]));
   prim[3] = fmaxr(prim[3], tiny);
   if (ph.cooling == COOL_NONE) {
-    T = quot(prim[3], dn);
+    T = divr(prim[3], r);
   } else if (ph.cooling == COOL_H) {
     R dentot = (R(2.) * r - prim[NEQ > 4 ? 4 : 0]);
     dentot = fmaxr(dentot, tiny);
     T = fmaxr(R(1.), divr(prim[3], dentot) * ph.tempsc);
     prim[3] = divr(dentot * T, ph.tempsc);
   } else {
-    T = fmaxr(R(1.), quot(prim[3], dn) * ph.tempsc);
+    T = fmaxr(R(1.), divr(prim[3], r) * ph.tempsc);
     prim[3] = divr(r * T, ph.tempsc);
   }
-}
-template <int NEQ, typename R>
-__device__ __forceinline__ void uprim(const Phys<R>& ph, R* prim, const R* uu, R& T)
-{
-  typename DenOf<R>::T dn;
-  uprim<NEQ>(ph, prim, uu, T, dn);
 }
 
 // src/primu.f90:4-19
@@ -145,7 +122,7 @@ __device__ __forceinline__ void primu(const Phys<R>& ph, const R* p, R* uu)
   uu[0] = p[0];
   uu[1] = p[0] * p[1];
   uu[2] = p[0] * p[2];
-  uu[3] = add_half(ph.cv * p[3], p[0] * (p[1] * p[1] + p[2] * p[2]));
+  uu[3] = kin_plus(p[0], p[1] * p[1] + p[2] * p[2], ph.cv * p[3]);
 #pragma unroll
   for (int k = 4; k < NEQ; ++k) uu[k] = p[k];
 }
@@ -154,7 +131,7 @@ __device__ __forceinline__ void primu(const Phys<R>& ph, const R* p, R* uu)
 template <int NEQ, typename R>
 __device__ __forceinline__ void primf(const Phys<R>& ph, const R* p, R* ff)
 {
-  R etot = add_half(ph.cv * p[3], p[0] * (p[1] * p[1] + p[2] * p[2]));
+  R etot = kin_plus(p[0], p[1] * p[1] + p[2] * p[2], ph.cv * p[3]);
   ff[0] = p[0] * p[1];
   ff[1] = p[0] * p[1] * p[1] + p[3];
   ff[2] = p[0] * p[1] * p[2];
@@ -166,30 +143,24 @@ __device__ __forceinline__ void primf(const Phys<R>& ph, const R* p, R* ff)
 // src/sound.f90:4-13
 template <typename R>
 __device__ __forceinline__ R sound(const Phys<R>& ph, R p, R d) { return sqrtr(divr(ph.gamma * p, d)); }
-// with the density as a divisor whose reciprocal is at hand
-template <typename R>
-__device__ __forceinline__ R sound(const Phys<R>& ph, R p, const typename DenOf<R>::T& dn)
-{
-  return sqrtr(quot(ph.gamma * p, dn));
-}
 
 // Star-region state of HLLC, src/hllcfluxes.f90:127-160, for the side
 // "s" (left: s = sl, smus = sl - u_l; right: s = sr, smus = sr - u_r).
 template <int NEQ, typename R>
-__device__ __forceinline__ void hllc_star(const Phys<R>& ph, const R* q, R s, R smus, R sst, R den,
-                                          const typename DenOf<R>::T& dn, R* ff)
+__device__ __forceinline__ void hllc_star(const Phys<R>& ph, const R* q, R s, R smus, R sst,
+                                          R den, R* ff)
 {
   // component by component (fewer values live at once), each term formed as
   // primf, primu and the star state form it: F + s (U* - U)
   const R rhost = divr(q[0] * smus, s - sst);
-  const R ek = add_half(ph.cv * q[3], q[0] * (q[1] * q[1] + q[2] * q[2]));
+  const R ek = kin_plus(q[0], q[1] * q[1] + q[2] * q[2], ph.cv * q[3]);
   ff[0] = q[0] * q[1] + s * (rhost - q[0]);
   ff[1] = (q[0] * q[1] * q[1] + q[3]) + s * (rhost * sst - q[0] * q[1]);
   ff[2] = q[0] * q[1] * q[2] + s * (rhost * q[2] - q[0] * q[2]);
   ff[3] = q[1] * (ek + q[3]) +
-          s * (rhost * (quot(ek, dn) + (sst - q[1]) * (sst + divr(q[3], den * smus))) - ek);
+          s * (rhost * (divr(ek, q[0]) + (sst - q[1]) * (sst + divr(q[3], den * smus))) - ek);
 #pragma unroll
-  for (int k = 4; k < NEQ; ++k) ff[k] = q[k] * q[1] + s * (quot(rhost * q[k], dn) - q[k]);
+  for (int k = 4; k < NEQ; ++k) ff[k] = q[k] * q[1] + s * (divr(rhost * q[k], q[0]) - q[k]);
 }
 
 // HLL flux between ql and qr, src/hllfluxes.f90:118-124
@@ -215,10 +186,8 @@ __device__ __forceinline__ void hll_flux(const Phys<R>& ph, const R* ql, const R
 // cell's sound speed pass it in; the value is the one sound() returns).
 // pl is overwritten (it holds the star side's state on return).
 // Returns false on the NaN contact speed that stops the reference.
-// dn(left, rho): that state's density as a divisor, asked for where the star
-// state is formed.
-template <int NEQ, typename R, typename D>
-__device__ __forceinline__ bool riemann(const Phys<R>& ph, R* pl, const R* pr, R csl, R csr, const D& dn, R* ff)
+template <int NEQ, typename R>
+__device__ __forceinline__ bool riemann(const Phys<R>& ph, R* pl, const R* pr, R csl, R csr, R* ff)
 {
   R beta1 = R(1.), beta2 = R(0.);
   if (ph.solver == SOLVER_HLL_HLLC) {              // hll_hllcfluxes.f90:110-129
@@ -255,7 +224,7 @@ __device__ __forceinline__ bool riemann(const Phys<R>& ph, R* pl, const R* pr, R
   const R den = left ? pl[0] : (ph.hllc_compat ? pr[3] : pr[0]);
 #pragma unroll
   for (int k = 0; k < NEQ; ++k) pl[k] = left ? pl[k] : pr[k];
-  hllc_star<NEQ>(ph, pl, left ? sl : sr, left ? slmul : srmur, sst, den, dn(left, pl[0]), ff);
+  hllc_star<NEQ>(ph, pl, left ? sl : sr, left ? slmul : srmur, sst, den, ff);
   if (ph.solver == SOLVER_HLL_HLLC) {
 #pragma unroll
     for (int k = 0; k < NEQ; ++k) ff[k] = beta1 * (ff[k]) + beta2 * (fh[k]);
