@@ -30,16 +30,6 @@
 
 using namespace w2d;
 
-// flat parameter vector: W1 [64 x 4], b1, W2 [64 x 64], b2, W3 [2 x 64], b3
-enum : int {
-  P_W1 = 0,
-  P_B1 = P_W1 + NN_H * NN_IN,
-  P_W2 = P_B1 + NN_H,
-  P_B2 = P_W2 + NN_H * NN_H,
-  P_W3 = P_B2 + NN_H,
-  P_B3 = P_W3 + NN_OUT * NN_H,
-  P_N = P_B3 + NN_OUT
-};
 static_assert(P_N == W2D_NN_NPARAM, "parameter count");
 
 struct W2dNN {
@@ -47,6 +37,7 @@ struct W2dNN {
   cudaStream_t st = nullptr;
   float* d_p = nullptr;      // fp32 master parameters
   float* d_g = nullptr;      // gradient (+1: loss)
+  float* d_part = nullptr;   // gradient slots of the batches of several tiles (first use allocates them)
   float* d_m = nullptr;      // Adam moments
   float* d_v = nullptr;
   NNImage* d_img = nullptr;  // bf16 operand image of d_p
@@ -245,34 +236,6 @@ struct __align__(128) NNTrainSmem {
   uint32_t tmem;
   int ok;
 };
-
-// TMEM columns
-constexpr int C_Z1 = 0, C_Z2 = 64, C_O = 128, C_G1 = 160, C_G3 = 192, C_G2 = 256, C_ALLOC = 512;
-
-// all threads: smem operands written, TMEM reads done -> MMA issue
-__device__ __forceinline__ void nn_sync()
-{
-  tc_fence_smem();
-  tc_fence_before();
-  __syncthreads();
-  tc_fence_after();
-}
-
-// all threads wait for the MMAs committed to bar (bounded); CTA-uniform
-// result.  On a timeout the error word is set and the wait is repeated once
-// (bounded) so that no MMA is still writing when the caller frees its TMEM.
-__device__ __forceinline__ bool nn_wait(uint64_t* bar, uint32_t& phase, int* err)
-{
-  const bool mine = mbar_wait(bar, phase);
-  if (!__syncthreads_and(mine)) {
-    if (threadIdx.x == 0) atomicExch(err, W2D_ERR_TIMEOUT);
-    mbar_wait(bar, phase);
-    return false;
-  }
-  phase ^= 1u;
-  tc_fence_after();
-  return true;
-}
 
 __device__ __forceinline__ void nn_ld64(uint32_t tm, int col, float* v)
 {
@@ -913,6 +876,30 @@ int nn_train_launch(W2dNN* nn, const float* feat, const float* targ, int64_t ld,
   return W2D_OK;
 }
 
+// `total` steps on batches of several tiles (w2d_nn_train.cu); the loss of the
+// last one is read once, behind them all
+int nn_train_multi(W2dNN* nn, int64_t total, int64_t steps_per_epoch, int batch, float lr, float lr_end,
+                   float* last_loss)
+{
+  if (!nn->d_part) NCK(cudaMalloc(&nn->d_part, sizeof(float) * nn_part_floats(nn->nsm)));
+  const NNTrainArgs a = {nn->d_p, nn->d_m, nn->d_v, nn->d_part, nn->d_img, nn->d_err, nn->nsm};
+  for (int64_t s = 0; s < total; ++s) {
+    // cosine decay from lr to lr_end
+    const double c = 0.5 * (1.0 + std::cos(std::acos(-1.0) * (double)s / (double)total));
+    const float lrs = (float)(lr_end + (lr - lr_end) * c);
+    nn->adam_t++;
+    const float b1c = 1.f - std::pow(0.9f, (float)nn->adam_t), b2c = 1.f - std::pow(0.999f, (float)nn->adam_t);
+    NCK(nn_train_step(a, nn->d_feat, nn->d_targ, nn->nsamp, (s % steps_per_epoch) * batch, batch, lrs, b1c, b2c,
+                      nn->st));
+  }
+  float loss = 0.f;
+  NCK(cudaMemcpyAsync(&loss, nn_train_loss(a), sizeof(float), cudaMemcpyDeviceToHost, nn->st));
+  int rc = nn_check(nn);
+  if (rc) return rc;
+  if (last_loss) *last_loss = loss;
+  return W2D_OK;
+}
+
 int nn_forward_launch(W2dNN* nn, const float* feat, int64_t ld, int64_t count, float* out)
 {
   static bool opted = false;
@@ -1031,7 +1018,7 @@ int w2d_nn_destroy(W2dNN* nn)
 {
   if (!nn) return W2D_ERR_ARG;
   if (nn->st) cudaStreamSynchronize(nn->st);
-  void* d[] = {nn->d_p, nn->d_g, nn->d_m, nn->d_v, nn->d_img, nn->d_err, nn->d_feat, nn->d_targ, nn->d_tab};
+  void* d[] = {nn->d_p, nn->d_g, nn->d_part, nn->d_m, nn->d_v, nn->d_img, nn->d_err, nn->d_feat, nn->d_targ, nn->d_tab};
   for (void* x : d)
     if (x) cudaFree(x);
   if (nn->st) cudaStreamDestroy(nn->st);
@@ -1091,6 +1078,7 @@ int w2d_nn_train(W2dNN* nn, int epochs, int batch, float lr, float lr_end, float
   const int64_t steps_per_epoch = nn->nsamp / batch;
   if (steps_per_epoch < 1) return W2D_ERR_ARG;
   const int64_t total = steps_per_epoch * epochs;
+  if (batch > 128) return nn_train_multi(nn, total, steps_per_epoch, batch, lr, lr_end, last_loss);
   double lsum = 0.0;
   int64_t lcount = 0;
   std::vector<float> h(P_N + 1);

@@ -29,6 +29,7 @@
 
 #include <cuda_bf16.h>
 
+#include "../../include/w2d.h"
 #include "w2d_tc.cuh"
 
 namespace w2d {
@@ -39,6 +40,17 @@ constexpr int NN_NOUT = 16;   // output N padded to the smallest M = 128 shape
 constexpr double NN_YR = 3.156e7;
 constexpr float NN_SY = 1e-16f, NN_AY = 22.f;
 constexpr float NN_W1 = 4.f;  // weight of the temperature-rate output in the training loss
+
+// flat parameter vector: W1 [64 x 4], b1, W2 [64 x 64], b2, W3 [2 x 64], b3
+enum : int {
+  P_W1 = 0,
+  P_B1 = P_W1 + NN_H * NN_IN,
+  P_W2 = P_B1 + NN_H,
+  P_B2 = P_W2 + NN_H * NN_H,
+  P_W3 = P_B2 + NN_H,
+  P_B3 = P_W3 + NN_OUT * NN_H,
+  P_N = P_B3 + NN_OUT
+};
 
 // bf16 images of the weights in the tensor-core operand layout (tc_off),
 // all K-major: W1 [64 x 16], W2 [64 x 64], W3 [16 x 64] (rows >= 2 zero),
@@ -232,5 +244,51 @@ __device__ __forceinline__ void nn_layer_mma(uint32_t tmem, int col, const uint1
   for (int k = 0; k < K / 16; ++k)
     tc_mma(tmem + (uint32_t)col, tc_desc(aa + 256u * k, 128u, sbo), tc_desc(bb + 256u * k, 128u, sbo), idesc, k > 0);
 }
+
+// TMEM columns
+constexpr int C_Z1 = 0, C_Z2 = 64, C_O = 128, C_G1 = 160, C_G3 = 192, C_G2 = 256, C_ALLOC = 512;
+
+// all threads: smem operands written, TMEM reads done -> MMA issue
+__device__ __forceinline__ void nn_sync()
+{
+  tc_fence_smem();
+  tc_fence_before();
+  __syncthreads();
+  tc_fence_after();
+}
+
+// all threads wait for the MMAs committed to bar (bounded); CTA-uniform
+// result.  On a timeout the error word is set and the wait is repeated once
+// (bounded) so that no MMA is still writing when the caller frees its TMEM.
+__device__ __forceinline__ bool nn_wait(uint64_t* bar, uint32_t& phase, int* err)
+{
+  const bool mine = mbar_wait(bar, phase);
+  if (!__syncthreads_and(mine)) {
+    if (threadIdx.x == 0) atomicExch(err, W2D_ERR_TIMEOUT);
+    mbar_wait(bar, phase);
+    return false;
+  }
+  phase ^= 1u;
+  tc_fence_after();
+  return true;
+}
+
+
+// Device arrays of a training run (w2d_nn_train.cu): parameters, Adam moments,
+// operand image, the CTAs' gradient slots (nn_part_floats) and the error word
+struct NNTrainArgs {
+  float *p, *m, *v, *part;
+  NNImage* img;
+  int* err;
+  int nsm;
+};
+size_t nn_part_floats(int nsm);
+// One training step on samples first .. first + count - 1 of feat, targ
+// (leading dimension ld): the gradient of their mean squared error and Adam with
+// rate lr and bias corrections b1c, b2c.
+cudaError_t nn_train_step(const NNTrainArgs& a, const float* feat, const float* targ, int64_t ld, int64_t first,
+                          int64_t count, float lr, float b1c, float b2c, cudaStream_t st);
+// where nn_train_step leaves the last step's loss
+const float* nn_train_loss(const NNTrainArgs& a);
 
 }  // namespace w2d
