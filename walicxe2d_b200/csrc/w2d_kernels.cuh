@@ -510,29 +510,6 @@ __device__ __forceinline__ double d_cooldmc(const double* __restrict__ tab, doub
   return (c1 - c0) * (T - T0) / (T1 - T0) + c0;
 }
 
-// Warp maximum of values >= 0 through the integer order of their bit patterns
-// (redux.sync: one instruction for a float, two and a select for a double,
-// against five shuffle rounds).  As fmax does, a NaN gives way to any number;
-// a warp of NaNs gives 0, or NaN with KEEP_NAN.
-template <bool KEEP_NAN = false>
-__device__ __forceinline__ double warp_max0(double x)
-{
-  const bool num = x >= 0.;
-  const unsigned hi = num ? (unsigned)__double2hiint(x) : 0u, lo = num ? (unsigned)__double2loint(x) : 0u;
-  const unsigned mh = __reduce_max_sync(0xffffffffu, hi);
-  const unsigned ml = __reduce_max_sync(0xffffffffu, hi == mh ? lo : 0u);
-  if (KEEP_NAN && !__any_sync(0xffffffffu, num)) return x;
-  return __hiloint2double((int)mh, (int)ml);
-}
-template <bool KEEP_NAN = false>
-__device__ __forceinline__ float warp_max0(float x)
-{
-  const bool num = x >= 0.f;
-  const unsigned m = __reduce_max_sync(0xffffffffu, num ? __float_as_uint(x) : 0u);
-  if (KEEP_NAN && !__any_sync(0xffffffffu, num)) return x;
-  return __uint_as_float(m);
-}
-
 // Per-block statistics of a primitive tile (cells 0..17 valid): the CFL
 // partial of timestep (src/timestep.f90:21-47), the criteria maximum
 // (src/criteria.f90:16-50) and, under DMC, the cooling-time limit.  Both

@@ -9,19 +9,22 @@
 //
 // This entry point computes it with the same arithmetic as w2d_timestep: a
 // per-block partial min(dx/(|u|+cs), dy/(|v|+cs)) over the interior cells,
-// then dt = min(cfl*min(partials), 0.4*1e30*Psc/tsc).  The partials live in
-// a file-scope device array of W2D_NOALLOC_MAX_BLOCKS doubles (512 KB, held
-// by every GPU that loads the library until the process exits); nothing is
-// allocated per call.  Built with --fmad=false like the FP64 kernels.
+// then dt = min(cfl*min(partials), 0.4*1e30*Psc/tsc).  The running minimum
+// lives in a file-scope device array of W2D_NOALLOC_MAX_BLOCKS doubles (512 KB,
+// held by every GPU that loads the library until the process exits); nothing
+// is allocated per call.  Built with --fmad=false like the FP64 kernels.
 #include <cuda_runtime.h>
+
+#include <algorithm>
 
 #include "../../include/w2d.h"
 #include "w2d_phys.cuh"
 
 namespace {
 
-// Per-block partials, then the result at index W2D_NOALLOC_MAX_BLOCKS and
-// the first block with a level outside 1..nlevs (0: none) at the index after.
+// [0] the complement of the least partial's bits, [1] of the first block (1
+// based) with a level outside 1..nlevs, [2] CTAs done (64-bit words, all zero
+// between calls); the results at W2D_NOALLOC_MAX_BLOCKS and the next index.
 static __device__ __align__(256) double g_noalloc_scratch[W2D_NOALLOC_MAX_BLOCKS + 32];
 
 struct Spacing {
@@ -29,76 +32,173 @@ struct Spacing {
   double dy[W2D_MAXLEV_NOALLOC + 1];
 };
 
-// A block whose level lies outside 1..nlevs gets the partial -(b+1): the
-// true partials are positive, so the reduction can tell them apart.
-template <int NEQ>
-__global__ void __launch_bounds__(256) k_cfl_partials(const double* __restrict__ u, const int32_t* __restrict__ lev,
-                                                      int nlevs, Spacing sp, w2d::Phys<double> ph,
-                                                      double* __restrict__ part)
+__device__ __forceinline__ float sqrt_near(float x)
 {
-  __shared__ double red[8];
-  const int b = blockIdx.x;
-  const int t = threadIdx.x;
-  const int i = 1 + t % 16, j = 1 + t / 16;
-  const double* ub = u + (size_t)b * NEQ * W2D_CELLS;
-  double uu[NEQ], q[NEQ], T;
-#pragma unroll
-  for (int k = 0; k < NEQ; ++k) uu[k] = ub[k * W2D_CELLS + (j + 1) * W2D_W + (i + 1)];
-  w2d::uprim<NEQ>(ph, q, uu, T);
-  const double cs = w2d::sound(ph, q[3], q[0]);
-  const int l = lev[b];
-  if (l < 1 || l > nlevs) {
-    if (t == 0) part[b] = -(double)(b + 1);
-    return;
-  }
-  const double t1 = sp.dx[l] / (fabs(q[1]) + cs);
-  const double t2 = sp.dy[l] / (fabs(q[2]) + cs);
-  // fmin here as in the reduction below: a NaN cell is ignored, as the
-  // context's max over |u|+cs ignores it
-  double m = fmin(t1, t2);
-#pragma unroll
-  for (int o = 16; o > 0; o >>= 1) m = fmin(m, __shfl_xor_sync(0xffffffffu, m, o));
-  if ((t & 31) == 0) red[t >> 5] = m;
-  __syncthreads();
-  if (t == 0) {
-    m = red[0];
-    for (int w = 1; w < 8; ++w) m = fmin(m, red[w]);
-    part[b] = m;
-  }
+  float y;
+  asm("sqrt.approx.f32 %0, %1;" : "=f"(y) : "f"(x));
+  return y;
 }
 
-__global__ void __launch_bounds__(1024) k_cfl_reduce(const double* __restrict__ part, int n, double courant,
-                                                     double psc, double tsc, double* __restrict__ out)
+// |u|+cs and |v|+cs of one cell, as k_dt's partials take them (NaN where the
+// cell's values give NaN)
+template <int NEQ>
+__device__ __forceinline__ void cell_speeds(const double* __restrict__ ub, int c, const w2d::Phys<double>& ph,
+                                            double& au, double& av)
 {
-  __shared__ double red[32], bad[32];
-  double m = 1.e30, worst = 0.0;   // worst: most negative partial (a bad level)
-  for (int k = threadIdx.x; k < n; k += blockDim.x) {
-    const double v = part[k];
-    if (v < 0.0) worst = fmin(worst, v);
-    else m = fmin(m, v);
-  }
+  double uu[NEQ], q[NEQ], T;
 #pragma unroll
-  for (int o = 16; o > 0; o >>= 1) {
-    m = fmin(m, __shfl_xor_sync(0xffffffffu, m, o));
-    worst = fmin(worst, __shfl_xor_sync(0xffffffffu, worst, o));
+  for (int k = 0; k < NEQ; ++k) uu[k] = ub[k * W2D_CELLS + c];
+  w2d::uprim<NEQ>(ph, q, uu, T);
+  const double cs = w2d::sound(ph, q[3], q[0]);
+  au = fabs(q[1]) + cs;
+  av = fabs(q[2]) + cs;
+}
+
+// Bounds of the same two speeds in FP32 (lo <= exact <= hi): the conversions,
+// products and roots below err by less than 1e-6 relative each, and the pressure
+// by less than 2e-6 of the energies it is the difference of.  Values whose
+// ranges or NaNs void that give (0, inf).
+struct Bounds {
+  float ulo, uhi, vlo, vhi;
+};
+template <bool H>
+__device__ __forceinline__ Bounds cell_bounds(double d0, double d1, double d2, double d3, double d4,
+                                              const w2d::Phys<double>& ph)
+{
+  const float r = fmaxf((float)d0, 1e-15f), mx = (float)d1, my = (float)d2, E = (float)d3;
+  const float inv = __fdividef(1.f, r), u = fabsf(mx * inv), v = fabsf(my * inv);
+  const float ke = 0.5f * (fabsf(mx) * u + fabsf(my) * v), er = 2e-6f * (fabsf(E) + ke);
+  const float icv = 1.f / (float)ph.cv, g = (float)ph.gamma * inv;
+  float plo = fmaxf((E - ke - er) * icv, 0.f), phi = fmaxf((E - ke + er) * icv, 1.1e-15f);
+  // coolingh: the pressure of T >= 1 (uprim)
+  if (H) phi = fmaxf(phi, 1.00001f * fmaxf(2.f * r - (float)d4, 1e-15f) / (float)ph.tempsc);
+  const float clo = sqrt_near(g * plo) * (1.f - 4e-6f), chi = sqrt_near(g * phi) * (1.f + 4e-6f);
+  const bool fit = ph.cv > 1e-3 && ph.cv < 1e3 && ph.gamma > 1e-3 && ph.gamma < 1e3 &&
+                   (!H || (ph.tempsc > 1e-12 && ph.tempsc < 1e30)) && r <= 1e15f && fabsf(E) <= 1e15f && fabsf(E) >= 1e-12f && fabsf(mx) <= 1e15f && fabsf(my) <= 1e15f &&
+                   (!H || fabs(d4) <= 1e15);
+  if (!fit) return {0.f, INFINITY, 0.f, INFINITY};
+  return {u * (1.f - 4e-6f) + clo, u * (1.f + 4e-6f) + chi, v * (1.f - 4e-6f) + clo, v * (1.f + 4e-6f) + chi};
+}
+
+// The minimum of the partials of the blocks this grid walks, a warp per block,
+// lane l taking cells 2 (l % 8) and the next of rows l / 8, 4 + l / 8, ... .
+// For a positive x, RN(dx/x) falls with x, so a block's partial needs only the
+// largest |u|+cs and |v|+cs.  FP32 bounds find the few cells that can hold
+// them (all 256 where a block is uniform); those alone are computed in FP64.
+// Bound by the blocks' bytes: 205 MB of sectors for 20,011 blocks of 4 equations
+// (every cell in FP64 with its own divisions, one CTA per block, a second kernel
+// for the minimum: 86 us a call; so 60, the kernel 41.5).  VEC: 16-byte loads (u on a 16-byte
+// boundary).
+template <int NEQ, bool H, bool VEC>
+__global__ void __launch_bounds__(256) k_cfl_min(const double* __restrict__ u, const int32_t* __restrict__ lev,
+                                                 int nblocks, int nlevs, Spacing sp, w2d::Phys<double> ph,
+                                                 double courant, double psc, double tsc,
+                                                 unsigned long long* __restrict__ work, double* __restrict__ out)
+{
+  __shared__ double red[8];
+  __shared__ int redb[8];
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+  const int at = (2 + lane / 8) * W2D_W + 2 + 2 * (lane % 8);   // first of the lane's cells in its first row
+  double m = 1.e30;
+  int bad = 0;                     // first block (1-based) with a bad level
+  for (int b = blockIdx.x * 8 + warp; b < nblocks; b += gridDim.x * 8) {
+    const double* ub = u + (size_t)b * NEQ * W2D_CELLS;
+    constexpr int NL = H && NEQ > 4 ? 5 : 4;   // (uprim takes the density where there is no fifth equation)
+    double x[4][NL][2];
+#pragma unroll
+    for (int k = 0; k < 4; ++k)
+#pragma unroll
+      for (int e = 0; e < NL; ++e) {
+        const double* p = ub + e * W2D_CELLS + at + k * 4 * W2D_W;
+        if (VEC) {
+          const double2 t = *reinterpret_cast<const double2*>(p);
+          x[k][e][0] = t.x;
+          x[k][e][1] = t.y;
+        } else {
+          x[k][e][0] = p[0];
+          x[k][e][1] = p[1];
+        }
+      }
+    const int l = lev[b];
+    if (l < 1 || l > nlevs) {
+      if (bad == 0) bad = b + 1;
+      continue;
+    }
+    float uhi[8], vhi[8], ulo = 0.f, vlo = 0.f;
+#pragma unroll
+    for (int c = 0; c < 8; ++c) {
+      const double(*y)[2] = x[c >> 1];
+      const int h = c & 1;
+      const Bounds z = cell_bounds<H>(y[0][h], y[1][h], y[2][h], y[3][h], H ? y[NL == 5 ? 4 : 0][h] : 0., ph);
+      uhi[c] = z.uhi;
+      vhi[c] = z.vhi;
+      ulo = fmaxf(ulo, z.ulo);
+      vlo = fmaxf(vlo, z.vlo);
+    }
+    ulo = __uint_as_float(__reduce_max_sync(0xffffffffu, __float_as_uint(ulo)));
+    vlo = __uint_as_float(__reduce_max_sync(0xffffffffu, __float_as_uint(vlo)));
+    unsigned cand = 0;
+#pragma unroll
+    for (int c = 0; c < 8; ++c) cand |= (unsigned)(!(uhi[c] < ulo) || !(vhi[c] < vlo)) << c;   // (NaN: a candidate)
+    double mu = 0., mv = 0.;
+    while (__any_sync(0xffffffffu, cand != 0)) {
+      if (cand) {
+        const int c = __ffs(cand) - 1;
+        cand &= cand - 1;
+        double au, av;
+        cell_speeds<NEQ>(ub, at + (c >> 1) * 4 * W2D_W + (c & 1), ph, au, av);
+        mu = fmax(mu, au);
+        mv = fmax(mv, av);
+      }
+    }
+    mu = w2d::warp_max0(mu);
+    mv = w2d::warp_max0(mv);
+    const double part = fmin(sp.dx[l] / mu, sp.dy[l] / mv);
+    if (part < 0.) {   // (a negative spacing)
+      if (bad == 0) bad = b + 1;
+      continue;
+    }
+    m = fmin(m, part + 0.);
   }
-  if ((threadIdx.x & 31) == 0) {
-    red[threadIdx.x >> 5] = m;
-    bad[threadIdx.x >> 5] = worst;
+  if (lane == 0) {
+    red[warp] = m;
+    redb[warp] = bad;
   }
   __syncthreads();
-  if (threadIdx.x == 0) {
-    m = red[0];
-    worst = bad[0];
-    for (int w = 1; w < 32; ++w) {
-      m = fmin(m, red[w]);
-      worst = fmin(worst, bad[w]);
-    }
-    const double a = courant * m;
-    const double c = 0.4 * 1e30 * psc / tsc;
-    out[0] = (a < c) ? a : c;
-    out[1] = -worst;   // a block ID + 1 with a bad level, or 0
+  if (threadIdx.x != 0) return;
+  for (int w = 1; w < 8; ++w) {
+    m = fmin(m, red[w]);
+    if (redb[w] && (!bad || redb[w] < bad)) bad = redb[w];
   }
+  // complements: zero is the neutral value of the maximum, and what the last
+  // CTA leaves behind (the partials are positive, so their bits order as they do)
+  atomicMax(&work[0], ~(unsigned long long)__double_as_longlong(m));
+  if (bad) atomicMax(&work[1], ~(unsigned long long)bad);
+  __threadfence();
+  if (atomicAdd(&work[2], 1ull) + 1ull != gridDim.x) return;
+  __threadfence();
+  m = __longlong_as_double((long long)~atomicExch(&work[0], 0ull));
+  const unsigned long long wb = atomicExch(&work[1], 0ull);
+  work[2] = 0ull;
+  const double a = courant * m;
+  const double c = 0.4 * 1e30 * psc / tsc;
+  out[0] = (a < c) ? a : c;
+  out[1] = wb ? (double)~wb : 0.;   // a block ID with a bad level, or 0
+}
+
+template <int NEQ, bool H>
+void launch_cfl(const double* u, const int32_t* lev, int nblocks, const W2dParams* p, const Spacing& sp,
+                const w2d::Phys<double>& ph, double* scratch)
+{
+  int dev = 0, nsm = 148;
+  if (cudaGetDevice(&dev) == cudaSuccess) cudaDeviceGetAttribute(&nsm, cudaDevAttrMultiProcessorCount, dev);
+  const int grid = std::min((nblocks + 7) / 8, 3 * nsm);   // three CTAs of 80 registers per SM
+  auto* work = reinterpret_cast<unsigned long long*>(scratch);
+  double* out = scratch + W2D_NOALLOC_MAX_BLOCKS;
+  if (((uintptr_t)u & 15) == 0)
+    k_cfl_min<NEQ, H, true><<<grid, 256>>>(u, lev, nblocks, p->nlevs, sp, ph, p->cfl, p->psc, p->tsc, work, out);
+  else
+    k_cfl_min<NEQ, H, false><<<grid, 256>>>(u, lev, nblocks, p->nlevs, sp, ph, p->cfl, p->psc, p->tsc, work, out);
 }
 
 // Device address of the scratch array in the caller's current device and
@@ -143,12 +243,21 @@ extern "C" int w2d_timestep_noalloc(const W2dParams* p, const double* u, const i
   ph.limiter = p->limiter;
   ph.cvh = ph.cvl = 0.0;
   ph.cv_split = w2d::cv_split(p->cv, &ph.cvh, &ph.cvl) ? 1 : 0;
+  const bool h = p->cooling == W2D_COOLINGH;
   switch (p->neq) {
-    case 4: k_cfl_partials<4><<<nblocks, 256>>>(u, lev, p->nlevs, sp, ph, scratch); break;
-    case 5: k_cfl_partials<5><<<nblocks, 256>>>(u, lev, p->nlevs, sp, ph, scratch); break;
-    default: k_cfl_partials<6><<<nblocks, 256>>>(u, lev, p->nlevs, sp, ph, scratch); break;
+    case 4:
+      if (h) launch_cfl<4, true>(u, lev, nblocks, p, sp, ph, scratch);
+      else launch_cfl<4, false>(u, lev, nblocks, p, sp, ph, scratch);
+      break;
+    case 5:
+      if (h) launch_cfl<5, true>(u, lev, nblocks, p, sp, ph, scratch);
+      else launch_cfl<5, false>(u, lev, nblocks, p, sp, ph, scratch);
+      break;
+    default:
+      if (h) launch_cfl<6, true>(u, lev, nblocks, p, sp, ph, scratch);
+      else launch_cfl<6, false>(u, lev, nblocks, p, sp, ph, scratch);
+      break;
   }
-  k_cfl_reduce<<<1, 1024>>>(scratch, nblocks, p->cfl, p->psc, p->tsc, scratch + W2D_NOALLOC_MAX_BLOCKS);
   if (cudaGetLastError() != cudaSuccess) return W2D_ERR_CUDA;
   double res[2];
   if (cudaMemcpy(res, scratch + W2D_NOALLOC_MAX_BLOCKS, sizeof(res), cudaMemcpyDeviceToHost) != cudaSuccess)

@@ -42,6 +42,29 @@ __device__ __forceinline__ double minus_kin(double y, double r, double v2) { ret
 __device__ __forceinline__ float kin_plus(float r, float v2, float y) { return 0.5f * r * v2 + y; }
 __device__ __forceinline__ float minus_kin(float y, float r, float v2) { return y - 0.5f * r * v2; }
 
+// Warp maximum of values >= 0 through the integer order of their bit patterns
+// (redux.sync: one instruction for a float, two and a select for a double,
+// against five shuffle rounds).  As fmax does, a NaN gives way to any number;
+// a warp of NaNs gives 0, or NaN with KEEP_NAN.
+template <bool KEEP_NAN = false>
+__device__ __forceinline__ double warp_max0(double x)
+{
+  const bool num = x >= 0.;
+  const unsigned hi = num ? (unsigned)__double2hiint(x) : 0u, lo = num ? (unsigned)__double2loint(x) : 0u;
+  const unsigned mh = __reduce_max_sync(0xffffffffu, hi);
+  const unsigned ml = __reduce_max_sync(0xffffffffu, hi == mh ? lo : 0u);
+  if (KEEP_NAN && !__any_sync(0xffffffffu, num)) return x;
+  return __hiloint2double((int)mh, (int)ml);
+}
+template <bool KEEP_NAN = false>
+__device__ __forceinline__ float warp_max0(float x)
+{
+  const bool num = x >= 0.f;
+  const unsigned m = __reduce_max_sync(0xffffffffu, num ? __float_as_uint(x) : 0u);
+  if (KEEP_NAN && !__any_sync(0xffffffffu, num)) return x;
+  return __uint_as_float(m);
+}
+
 enum { SOLVER_HLLC = 0, SOLVER_HLL = 1, SOLVER_HLL_HLLC = 2 };
 enum { COOL_NONE = 0, COOL_H = 1, COOL_DMC = 2 };
 
