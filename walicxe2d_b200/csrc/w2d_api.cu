@@ -111,11 +111,14 @@ constexpr int kNShape = (int)(sizeof(kShapes) / sizeof(kShapes[0]));
 // CTAs per SM of a shape's persistent grid.  The cooling kernel holds three
 // per SM (64 registers, 320 threads): its grids of 4 and 8 would leave the
 // last wave a third full (FP32 ensemble of 6,641 leaves: 151 us on 4 per SM,
-// 130 on 3; compiled for 2 per SM 137).
+// 130 on 3; compiled for 2 per SM 137).  Fill I holds three in FP64 with the
+// criteria: two waves of them in place of 4 (3,385 leaves: 21.0 us on 4 per SM,
+// 20.9 on 3, 19.2 on 6; 8,835: 41.5, 39.6, 39.3).
 int shape_per_sm(int sh, int tk)
 {
   const int per = kShapes[sh].per_sm;
-  return tk == TK_COOL && per >= 4 ? per * 3 / 4 : per;
+  if (tk == TK_COOL && per >= 4) return per * 3 / 4;
+  return tk == TK_FILL1 && per == 4 ? 6 : per;
 }
 
 void apply_shape(W2dCtx* c, KArgs& a, int tk)

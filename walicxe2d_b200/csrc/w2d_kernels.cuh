@@ -989,11 +989,19 @@ __device__ __forceinline__ void fill1_leaf(const KArgs& a, const PhysArgs& pa, c
   const int cj = gj < 1 ? 1 : (gj > W2D_NX ? W2D_NX : gj);
   const int b = a.leaves[li];
   const int2 d = fd[li * 4 + f];
-  R gv[NEQ];
+  R* __restrict__ u = upool + (size_t)b * bs;
+  // every load is issued before the first store: the edge cell's values do not
+  // wait for the gather (a store to the pool would order them behind it).  Fill
+  // I on 8,835 blocks 53.6 -> 41.3 us, at 74 registers; capped to 64 for a
+  // fourth CTA per SM 70 us.
+  R gv[NEQ], uc[NEQ];
   bool w = false;
 #pragma unroll
   for (int k = 0; k < NEQ; ++k) w = ghost_value<R>(upool, bs, a, b, d, f, 0, m, k, gv[k]);
-  R* __restrict__ u = upool + (size_t)b * bs;
+  if (a.split_stats) {
+#pragma unroll
+    for (int k = 0; k < NEQ; ++k) uc[k] = u[k * W2D_CELLS + cidx(ci, cj)];
+  }
   if (w) {
 #pragma unroll
     for (int k = 0; k < NEQ; ++k) u[k * W2D_CELLS + cidx(gi, gj)] = gv[k];
@@ -1003,11 +1011,10 @@ __device__ __forceinline__ void fill1_leaf(const KArgs& a, const PhysArgs& pa, c
   // primitives of both as calcprim gives them; a face no entry writes
   // keeps the ghost value it has
   const Phys<R> ph = make_phys<R, -1, -1>(pa);
-  R uc[NEQ], qc[NEQ], qg[NEQ], T;
+  R qc[NEQ], qg[NEQ], T;
+  if (!w) {
 #pragma unroll
-  for (int k = 0; k < NEQ; ++k) {
-    if (!w) gv[k] = u[k * W2D_CELLS + cidx(gi, gj)];
-    uc[k] = u[k * W2D_CELLS + cidx(ci, cj)];
+    for (int k = 0; k < NEQ; ++k) gv[k] = u[k * W2D_CELLS + cidx(gi, gj)];
   }
   uprim<NEQ>(ph, qg, gv, T);
   uprim<NEQ>(ph, qc, uc, T);
