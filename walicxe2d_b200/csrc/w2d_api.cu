@@ -114,9 +114,11 @@ constexpr int kNShape = (int)(sizeof(kShapes) / sizeof(kShapes[0]));
 // 130 on 3; compiled for 2 per SM 137).  Fill I holds three in FP64 with the
 // criteria: two waves of them in place of 4 (3,385 leaves: 21.0 us on 4 per SM,
 // 20.9 on 3, 19.2 on 6; 8,835: 41.5, 39.6, 39.3).
-int shape_per_sm(int sh, int tk)
+// The half and full steps' grids of 4 and 8 become 3 and 6 where 3 CTAs fit.
+int shape_per_sm(const W2dCtx* c, int sh, int tk)
 {
   const int per = kShapes[sh].per_sm;
+  if ((tk == TK_HALF || tk == TK_FULL) && per >= 4) return per / 4 * step_ctas(tk == TK_FULL, c->neq, c->elem);
   if (tk == TK_COOL && per >= 4) return per * 3 / 4;
   return tk == TK_FILL1 && per == 4 ? 6 : per;
 }
@@ -124,7 +126,7 @@ int shape_per_sm(int sh, int tk)
 void apply_shape(W2dCtx* c, KArgs& a, int tk)
 {
   const int sh = c->tune_left > 0 ? c->tune_cur : c->tshape[tk];
-  a.grid = shape_per_sm(sh, tk) * c->nsm;
+  a.grid = shape_per_sm(c, sh, tk) * c->nsm;
   a.sched = kShapes[sh].sched;
 }
 
@@ -2147,7 +2149,7 @@ int w2d_tuning(W2dCtx* c, int32_t* shape, double* ms, int* tuning_left)
     const int sh = c->tshape[k];
     if (shape) {
       shape[3 * k] = sh;
-      shape[3 * k + 1] = shape_per_sm(sh, k);
+      shape[3 * k + 1] = shape_per_sm(c, sh, k);
       shape[3 * k + 2] = kShapes[sh].sched;
     }
     if (ms) ms[k] = c->tune_n[k][sh] > 0 ? c->tune_ms[k][sh] / c->tune_n[k][sh] : 0.0;

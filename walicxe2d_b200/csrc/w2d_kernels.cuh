@@ -442,16 +442,19 @@ __device__ __forceinline__ bool wait_tiles(uint64_t* bar, int* err, int b)
 
 // CTAs per SM the per-leaf kernels are compiled for: 4, i.e. at most 56
 // registers per thread at 288 threads.  In FP64 the half and full steps
-// then spill a few registers (about 60 and 110 bytes of spill loads) but
-// keep 4 CTAs (36 warps) per SM instead of 3, which measured 12% (half) and
-// 7% (full) faster: the FP64 pipe waits less on the long division and
-// square-root chains.  In FP32, 5 and 6 CTAs
-// per SM (40 and 32 registers, 150-210 bytes of spill loads in the full
-// step) measured 3% and 13% slower on the 256-run ensemble than 4.
-template <typename R>
-__host__ __device__ constexpr int w2d_minb(bool)
+// then spill a few registers but keep 4 CTAs (36 warps) per SM instead of 3,
+// which measured 12% (half) and 7% (full) faster: the FP64 pipe waits less on
+// the long division and square-root chains.  In FP32, 5 and 6 CTAs per SM (40
+// and 32 registers, 150-210 bytes of spill loads in the full step) measured 3%
+// and 13% slower on the 256-run ensemble than 4.  Where the shared memory of 4
+// does not fit an SM (FP64: 6 equations, and the half step's 5), 3 get 72
+// registers and a grid of their own number (step_ctas): FP64 remnant of 2,080
+// leaves, 6 equations, full step 82 -> 64 us, half step 48 -> 39 us against 56
+// registers on a grid of 4 per SM, whose last wave was a third full.
+constexpr int fit_ctas(size_t smem)
 {
-  return 4;
+  const int n = (int)(228 * 1024 / (smem + 1024));
+  return n < 1 ? 1 : n > 4 ? 4 : n;
 }
 
 // Tile copies of the persistent kernels: the barrier is initialised once per
@@ -788,7 +791,7 @@ __device__ __forceinline__ bool half_leaf(const KArgs& a, const PhysArgs& pa, do
 }
 
 template <typename R, int NEQ, int SOLVER, bool P>
-__global__ void __launch_bounds__(W2D_THREADS, w2d_minb<R>(P)) k_half(KArgs a, PhysArgs pa, double dt)
+__global__ void __launch_bounds__(W2D_THREADS, fit_ctas(smem_half<R, NEQ>())) k_half(KArgs a, PhysArgs pa, double dt)
 {
   bar_init_once(reinterpret_cast<uint64_t*>(w2d_smem));
   pdl_begin();
@@ -954,8 +957,18 @@ __device__ __forceinline__ bool full_leaf(const KArgs& a, const PhysArgs& pa, do
   return true;
 }
 
+// CTAs of the half step (full: of the full step) an SM holds
+inline int step_ctas(bool full, int neq, size_t elem)
+{
+  const size_t tiles = 2 * (size_t)neq * W2D_CELLS, fluxes = 2 * (size_t)neq * 272;
+  return fit_ctas(full ? 128 + 192 + elem * (tiles + fluxes) : 128 + elem * (tiles + W2D_CELLS + fluxes));
+}
+static_assert(smem_full<double, 6>() == 128 + 192 + 8 * (2 * 6 * W2D_CELLS + 2 * 6 * 272) &&
+                  smem_half<float, 5>() == 128 + 4 * (2 * 5 * W2D_CELLS + W2D_CELLS + 2 * 5 * 272),
+              "step_ctas");
+
 template <typename R, int NEQ, int SOLVER, int LIMITER, bool P>
-__global__ void __launch_bounds__(W2D_THREADS, w2d_minb<R>(P)) k_full(KArgs a, PhysArgs pa, double dt)
+__global__ void __launch_bounds__(W2D_THREADS, fit_ctas(smem_full<R, NEQ>())) k_full(KArgs a, PhysArgs pa, double dt)
 {
   bar_init_once(reinterpret_cast<uint64_t*>(w2d_smem));
   pdl_begin();
@@ -1062,7 +1075,7 @@ __host__ __device__ constexpr size_t smem_calcprim()
 // (coolingdmc, after cooling): the statistics of the stored primitives of
 // cells 0..17, which the cooling step wrote, without recomputing them.
 template <typename R, int NEQ, bool P>
-__global__ void __launch_bounds__(W2D_THREADS, w2d_minb<R>(P)) k_calcprim(KArgs a, PhysArgs pa,
+__global__ void __launch_bounds__(W2D_THREADS, 4) k_calcprim(KArgs a, PhysArgs pa,
                                                                          const int* __restrict__ list, int n,
                                                                          int mode)
 {
