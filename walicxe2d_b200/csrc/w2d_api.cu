@@ -305,6 +305,18 @@ int ensure_stage(W2dCtx* c, size_t bytes)
 // blocks per chunk of a staged transfer
 int stage_chunk(const W2dCtx* c) { return (int)std::max<size_t>(1, c->stage_bytes / (c->bs * sizeof(double))); }
 
+// bytes per flag plane: cap+1 rounded up, so that every plane starts on a
+// 256-byte boundary (k_admesh_flags sets flags with 32-bit atomics)
+size_t mark_plane(const W2dCtx* c) { return ((size_t)c->cap + 1 + 255) & ~(size_t)255; }
+
+// both sets of admesh's flag planes and the list counters back to zero
+void mark_reset(W2dCtx* c)
+{
+  if (!c->d_mflags || !c->d_mlists) return;
+  cudaMemsetAsync(c->d_mflags, 0, 6 * mark_plane(c), c->st);
+  cudaMemsetAsync(c->d_mlists, 0, 4 * sizeof(int), c->st);
+}
+
 // Checks the device error word (the queue must have drained).
 int check_device(W2dCtx* c)
 {
@@ -319,6 +331,7 @@ int check_device(W2dCtx* c)
     // a grid barrier that ran out left its count behind
     if (c->d_gbar) cudaMemsetAsync(c->d_gbar, 0, 2 * sizeof(unsigned int), c->st);
     c->gbar_count = 0;
+    mark_reset(c);   // so may a flags launch that gave up
     // so may the fused step's; its flags restart with its epoch
     if (c->d_step_sync) {
       cudaMemsetAsync(c->d_step_sync, 0, 4 * sizeof(unsigned), c->st);
@@ -1286,9 +1299,6 @@ int w2d_criteria(W2dCtx* c, double* grad)
 
 namespace {
 
-// bytes per flag plane: cap+1 rounded up, so that every plane starts on a
-// 256-byte boundary (k_markref_up sets flags with 32-bit atomics)
-size_t mark_plane(const W2dCtx* c) { return ((size_t)c->cap + 1 + 255) & ~(size_t)255; }
 
 // The device side of the admesh flags, allocated on first use (contexts
 // whose host takes the flags from w2d_criteria never hold it).
@@ -1298,8 +1308,9 @@ int ensure_mark(W2dCtx* c)
   const size_t slots = (size_t)c->cap + 1;
   CK(cudaMalloc(&c->d_links, sizeof(int4) * slots));
   CK(cudaMalloc(&c->d_sons, sizeof(int2) * slots));
-  CK(cudaMalloc(&c->d_mflags, 3 * mark_plane(c)));
+  CK(cudaMalloc(&c->d_mflags, 6 * mark_plane(c)));
   CK(cudaMalloc(&c->d_mlists, sizeof(int) * (4 + 2 * slots)));
+  mark_reset(c);
   CK(cudaMalloc(&c->d_rows7, sizeof(int) * 7 * slots));
   CK(cudaMallocHost(&c->h_mlists, sizeof(int) * (4 + 2 * slots)));
   CK(cudaMallocHost(&c->h_rows7, sizeof(int) * 7 * slots));
@@ -1427,15 +1438,28 @@ int w2d_admesh_flags(W2dCtx* c, int32_t* refine, int cap_refine, int* nrefine, i
   a.grad = c->d_grad;
   a.tol = c->p.tol;
   a.tol2 = c->p.tol2;
-  a.leafp = c->d_mflags;
-  a.up = c->d_mflags + plane;
-  a.down = c->d_mflags + 2 * plane;
+  unsigned char* set = c->d_mflags + 3 * plane * (size_t)c->mark_set;
+  c->mark_set ^= 1;
+  a.leafp = set;
+  a.up = set + plane;
+  a.down = set + 2 * plane;
+  a.next = c->d_mflags + 3 * plane * (size_t)c->mark_set;
+  // the counters and the heads of both lists in one wait; longer lists
+  // (rare: a pass that remeshes thousands of blocks) in a second one
+  const int head = (int)std::min<size_t>(slots, 2048);
+  int* h = c->h_mlists;
+  h[2] = 0;
+  a.done = c->d_gbar + 1;
+  a.host = h;
+  a.head = head;
+  a.slots = (int)slots;
+  a.err_host = c->h_err;
   a.counts = c->d_mlists;
   a.rlist = c->d_mlists + 4;
   a.clist = c->d_mlists + 4 + slots;
   a.err = c->d_err;
-  // the planes and counters zeroed, markref + critneighup, then the refine
-  // list, critneighdown and the coarsened families: one launch
+  // markref + critneighup, then the refine list, critneighdown and the
+  // coarsened families: one launch
   int rc = launch(c, "admesh_flags", [&] {
     unsigned int n = 0;
     const cudaError_t e = launch_admesh_flags(a, plane, c->d_gbar, c->gbar_count, &n, c->st);
@@ -1443,14 +1467,12 @@ int w2d_admesh_flags(W2dCtx* c, int32_t* refine, int cap_refine, int* nrefine, i
     return e;
   });
   if (rc) return rc;
-  // the counters and the heads of both lists in one wait; longer lists
-  // (rare: a pass that remeshes thousands of blocks) in a second one
-  const int head = (int)std::min<size_t>(slots, 2048);
-  int* h = c->h_mlists;
-  CK(cudaMemcpyAsync(h, c->d_mlists, sizeof(int) * (4 + (size_t)head), cudaMemcpyDeviceToHost, c->st));
-  CK(cudaMemcpyAsync(h + 4 + slots, c->d_mlists + 4 + slots, sizeof(int) * (size_t)head, cudaMemcpyDeviceToHost,
-                     c->st));
-  if ((rc = sync_and_check(c))) return rc;
+  CK(cudaStreamSynchronize(c->st));
+  tune_collect(c);
+  // (a launch whose barrier gave up handed nothing over: the error word says so)
+  if (h[2] == 0) CK(cudaMemcpy(c->h_err, c->d_err, 4 * sizeof(int), cudaMemcpyDeviceToHost));
+  if ((rc = check_device(c))) return rc;
+  if (h[2] == 0) return set_error(c, W2D_ERR_TIMEOUT, 0, 0, 0, "admesh flags: no lists");
   const int nr = std::min(h[0], (int)slots), nc = std::min(h[1], (int)slots);
   if (nr > head || nc > head) {
     if (nr > head)

@@ -124,11 +124,12 @@ struct W2dCtx {
   cudaEvent_t ev_plan[2] = {nullptr, nullptr};
   int plan_buf = 0;
   // admesh flags on the device (allocated by the first w2d_set_links): the
-  // mirror of lp(:,3:8), three byte planes of cap+1 flags, the two lists
+  // mirror of lp(:,3:8), two sets of three byte planes of cap+1 flags, the two lists
   // behind two counters, and the pinned row staging of w2d_set_links
   int4* d_links = nullptr;
   int2* d_sons = nullptr;     // lp(:,3), lp(:,4)
-  unsigned char* d_mflags = nullptr;
+  unsigned char* d_mflags = nullptr;   // two sets of the three planes
+  int mark_set = 0;                    // the set of the next call
   int* d_mlists = nullptr;    // [4 counters][cap+1 refines][cap+1 first sons]
   int* h_mlists = nullptr;    // pinned, same layout
   int* d_rows7 = nullptr;     // (nb, lp(nb,3:8)) per row, cap+1 rows

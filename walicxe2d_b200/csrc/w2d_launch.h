@@ -92,9 +92,13 @@ cudaError_t launch_dt_runs(const int* leaves, const int* loff, int nruns, const 
 // admesh flags on the device (w2d_mark.cu).  Per slot: lev, the mirror of
 // lp(:,3:4) (sons: first son, son position) and lp(:,5:8) (links), the
 // criteria maximum grad; byte
-// planes leafp, up, down zeroed before markref; counts[0..1] the
-// lengths of rlist (refines) and clist (first sons of coarsened families),
-// zeroed before, in atomic order.
+// planes leafp, up, down zero on entry (next: the other set of three, which the
+// launch zeroes for the call after it); counts[0..1] the lengths of rlist
+// (refines) and clist (first sons of coarsened families), in atomic order, zero
+// on entry and left zero.  The last CTA (done, zero on entry and left zero)
+// stores the counts to host[0..1], the first `head` entries of the lists behind
+// host + 4 and host + 4 + slots, the error word to err_host, and 1 to host[2]
+// (pinned memory).
 struct MarkArgs {
   const int* leaves;
   int nleaf, nbmax, cap, nlevs;
@@ -107,11 +111,15 @@ struct MarkArgs {
   int* counts;
   int* rlist;
   int* clist;
+  unsigned char* next;
+  unsigned int* done;
+  int* host;
+  int head, slots;
+  int* err_host;
   int* err;      // the context's error word (W2D_ERR_TOPOLOGY on a malformed tree)
 };
-// the flag planes and counts zeroed, markref with the whole critneighup
-// cascade, then the refine list, critneighdown and the coarsened families:
-// one cooperative launch
+// markref with the whole critneighup cascade, then the refine list,
+// critneighdown and the coarsened families: one cooperative launch
 // bar_base: the barrier count when the launch begins; *arrivals: the count
 // it adds (the host keeps the running count)
 cudaError_t launch_admesh_flags(const MarkArgs& a, size_t plane_bytes, unsigned int* bar, unsigned int bar_base,

@@ -534,21 +534,43 @@ __global__ void __launch_bounds__(kThreads) k_flag_leaves(const int* __restrict_
 }
 
 // ---- admesh flags in one launch ------------------------------------------------
-// The three flag planes and the list counters zeroed, markref with the
-// critneighup closure, then the refine list, critneighdown and the
-// coarsened families, with a barrier between the phases.
+// markref with the critneighup closure, a barrier, then the refine list,
+// critneighdown and the coarsened families; the last CTA hands the lists over.
+// The launch zeroes the next call's planes beside its own work (zeroing its own
+// first cost a barrier more), and the stores to pinned memory replace three
+// copies behind it.
 __global__ void __launch_bounds__(kThreads) k_admesh_flags(MarkArgs a, size_t plane_words, unsigned int* bar,
                                                            unsigned int bar_base)
 {
-  const int gtid = blockIdx.x * blockDim.x + threadIdx.x, gsz = gridDim.x * blockDim.x;
+  __shared__ bool last;
+  const int tid = threadIdx.x;
+  const int gtid = blockIdx.x * blockDim.x + tid, gsz = gridDim.x * blockDim.x;
   const GridBar gb{bar, bar_base, a.err};
-  unsigned int* w = reinterpret_cast<unsigned int*>(a.leafp);   // leafp, up, down are contiguous
-  for (size_t k = gtid; k < 3 * plane_words; k += gsz) w[k] = 0u;
-  if (gtid < 4) a.counts[gtid] = 0;
-  if (!grid_barrier(gb, 1)) return;
   for (int k = gtid; k < a.nleaf; k += gsz) markref_up_one(a, k);
-  if (!grid_barrier(gb, 2)) return;
+  unsigned int* w = reinterpret_cast<unsigned int*>(a.next);   // three planes in a row
+  for (size_t k = gtid; k < 3 * plane_words; k += gsz) w[k] = 0u;
+  if (!grid_barrier(gb, 1)) return;
   for (int nb = 1 + gtid; nb <= a.nbmax; nb += gsz) refine_coarsen_one(a, nb);
+  __syncthreads();
+  if (tid == 0) {
+    __threadfence();
+    last = atomicAdd(a.done, 1u) + 1u == gridDim.x;
+  }
+  __syncthreads();
+  if (!last) return;
+  __threadfence();
+  const int nr = __ldcg(a.counts), nc = __ldcg(a.counts + 1);
+  for (int k = tid; k < nr && k < a.head; k += blockDim.x) a.host[4 + k] = __ldcg(a.rlist + k);
+  for (int k = tid; k < nc && k < a.head; k += blockDim.x) a.host[4 + a.slots + k] = __ldcg(a.clist + k);
+  if (tid < 4) a.err_host[tid] = __ldcg(a.err + tid);
+  __syncthreads();
+  if (tid == 0) {
+    a.counts[0] = a.counts[1] = 0;
+    *a.done = 0u;
+    a.host[0] = nr;
+    a.host[1] = nc;
+    a.host[2] = 1;
+  }
 }
 
 inline int ctas(int n) { return (n + kThreads - 1) / kThreads; }
@@ -630,7 +652,7 @@ cudaError_t launch_admesh_flags(const MarkArgs& a, size_t plane_bytes, unsigned 
   void* args[] = {&marg, &w, &b, &base};
   const cudaError_t e =
       cudaLaunchCooperativeKernel((const void*)k_admesh_flags, dim3(grid), dim3(kThreads), args, 0, st);
-  if (e == cudaSuccess) *arrivals = 2u * (unsigned int)grid;
+  if (e == cudaSuccess) *arrivals = (unsigned int)grid;
   return e;
 }
 
