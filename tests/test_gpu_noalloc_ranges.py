@@ -93,3 +93,22 @@ def test_noalloc_refuses_and_recovers():
     lev[40] = 2
     assert _call(p, u, lev, -dx)[0] == 5
     assert _call(p, u, lev, dx) == (0, _exact(p, u, lev, dx))
+
+
+@pytest.mark.parametrize("kind", ["plain", "extreme"])
+@pytest.mark.parametrize("past", [0, 1, 9])
+def test_noalloc_around_one_block_per_cta(kind, past):
+    import torch
+    n = 4 * torch.cuda.get_device_properties(0).multi_processor_count + past
+    rng = np.random.default_rng([n, len(kind)])
+    p = base_params(neq=5, npas=1, nlevs=4, cooling=COOLINGH)
+    dx = np.array([0.1, 0.05, 0.025, 0.0125])
+    u = _state(kind, n, 5, rng)
+    lev = rng.integers(1, 5, n).astype(np.int32)
+    want = _exact(p, u, lev, dx)
+    assert _call(p, u, lev, dx) == (0, want)
+    keep = lev[n - 1]
+    lev[n - 1] = 5                    # W2D_ERR_TOPOLOGY, dt untouched
+    assert _call(p, u, lev, dx) == (5, -1.0)
+    lev[n - 1] = keep
+    assert _call(p, u, lev, dx) == (0, want)

@@ -80,6 +80,66 @@ __device__ __forceinline__ Bounds cell_bounds(double d0, double d1, double d2, d
   return {u * (1.f - 4e-6f) + clo, u * (1.f + 4e-6f) + chi, v * (1.f - 4e-6f) + clo, v * (1.f + 4e-6f) + chi};
 }
 
+// A CTA's minimum and first bad block into the words; the last CTA of the grid
+// writes the results and leaves the words zero.  One thread of a CTA.
+__device__ __forceinline__ void cfl_finish(double m, int bad, double courant, double psc, double tsc,
+                                           unsigned long long* __restrict__ work, double* __restrict__ out)
+{
+  // complements: zero is the neutral value of the maximum, and what the last
+  // CTA leaves behind (the partials are positive, so their bits order as they do)
+  atomicMax(&work[0], ~(unsigned long long)__double_as_longlong(m));
+  if (bad) atomicMax(&work[1], ~(unsigned long long)bad);
+  __threadfence();
+  if (atomicAdd(&work[2], 1ull) + 1ull != gridDim.x) return;
+  __threadfence();
+  m = __longlong_as_double((long long)~atomicExch(&work[0], 0ull));
+  const unsigned long long wb = atomicExch(&work[1], 0ull);
+  work[2] = 0ull;
+  const double a = courant * m;
+  const double c = 0.4 * 1e30 * psc / tsc;
+  out[0] = (a < c) ? a : c;
+  out[1] = wb ? (double)~wb : 0.;   // a block ID with a bad level, or 0
+}
+
+// One block per CTA, a thread per cell, every cell in FP64: the shorter chain
+// (one load, no bounds to rank) where the CTAs of the whole call are resident at
+// once.  500 blocks are 26 us a call, of which the launch and the copy of the
+// result are nearly all (28 with a second kernel for the minimum).
+template <int NEQ>
+__global__ void __launch_bounds__(256) k_cfl_few(const double* __restrict__ u, const int32_t* __restrict__ lev,
+                                                 int nlevs, Spacing sp, w2d::Phys<double> ph, double courant,
+                                                 double psc, double tsc, unsigned long long* __restrict__ work,
+                                                 double* __restrict__ out)
+{
+  __shared__ double red[2][8];
+  const int b = blockIdx.x, t = threadIdx.x;
+  const int l = lev[b];
+  double au, av;
+  cell_speeds<NEQ>(u + (size_t)b * NEQ * W2D_CELLS, (2 + t / 16) * W2D_W + 2 + t % 16, ph, au, av);
+  au = w2d::warp_max0(fmax(au, 0.));   // (NaN: left out)
+  av = w2d::warp_max0(fmax(av, 0.));
+  if ((t & 31) == 0) {
+    red[0][t >> 5] = au;
+    red[1][t >> 5] = av;
+  }
+  __syncthreads();
+  if (t != 0) return;
+  for (int w = 1; w < 8; ++w) {
+    au = fmax(au, red[0][w]);
+    av = fmax(av, red[1][w]);
+  }
+  double m = 1.e30;
+  int bad = b + 1;
+  if (l >= 1 && l <= nlevs) {
+    const double part = fmin(sp.dx[l] / au, sp.dy[l] / av);
+    if (!(part < 0.)) {   // (a negative spacing)
+      m = fmin(m, part + 0.);
+      bad = 0;
+    }
+  }
+  cfl_finish(m, bad, courant, psc, tsc, work, out);
+}
+
 // The minimum of the partials of the blocks this grid walks, a warp per block,
 // lane l taking cells 2 (l % 8) and the next of rows l / 8, 4 + l / 8, ... .
 // For a positive x, RN(dx/x) falls with x, so a block's partial needs only the
@@ -170,20 +230,7 @@ __global__ void __launch_bounds__(256) k_cfl_min(const double* __restrict__ u, c
     m = fmin(m, red[w]);
     if (redb[w] && (!bad || redb[w] < bad)) bad = redb[w];
   }
-  // complements: zero is the neutral value of the maximum, and what the last
-  // CTA leaves behind (the partials are positive, so their bits order as they do)
-  atomicMax(&work[0], ~(unsigned long long)__double_as_longlong(m));
-  if (bad) atomicMax(&work[1], ~(unsigned long long)bad);
-  __threadfence();
-  if (atomicAdd(&work[2], 1ull) + 1ull != gridDim.x) return;
-  __threadfence();
-  m = __longlong_as_double((long long)~atomicExch(&work[0], 0ull));
-  const unsigned long long wb = atomicExch(&work[1], 0ull);
-  work[2] = 0ull;
-  const double a = courant * m;
-  const double c = 0.4 * 1e30 * psc / tsc;
-  out[0] = (a < c) ? a : c;
-  out[1] = wb ? (double)~wb : 0.;   // a block ID with a bad level, or 0
+  cfl_finish(m, bad, courant, psc, tsc, work, out);
 }
 
 template <int NEQ, bool H>
@@ -192,9 +239,16 @@ void launch_cfl(const double* u, const int32_t* lev, int nblocks, const W2dParam
 {
   int dev = 0, nsm = 148;
   if (cudaGetDevice(&dev) == cudaSuccess) cudaDeviceGetAttribute(&nsm, cudaDevAttrMultiProcessorCount, dev);
-  const int grid = std::min((nblocks + 7) / 8, 3 * nsm);   // three CTAs of 80 registers per SM
   auto* work = reinterpret_cast<unsigned long long*>(scratch);
   double* out = scratch + W2D_NOALLOC_MAX_BLOCKS;
+  // Up to four CTAs per SM of one block each.  A call in us, k_cfl_few and
+  // k_cfl_min: 500 blocks 26 and 32, 1,000 and 2,500 33 and 32 each, 5,000 35
+  // and 33, 20,011 72 and 61.
+  if (nblocks <= 4 * nsm) {
+    k_cfl_few<NEQ><<<nblocks, 256>>>(u, lev, p->nlevs, sp, ph, p->cfl, p->psc, p->tsc, work, out);
+    return;
+  }
+  const int grid = std::min((nblocks + 7) / 8, 3 * nsm);   // three CTAs of 80 registers per SM
   if (((uintptr_t)u & 15) == 0)
     k_cfl_min<NEQ, H, true><<<grid, 256>>>(u, lev, nblocks, p->nlevs, sp, ph, p->cfl, p->psc, p->tsc, work, out);
   else
