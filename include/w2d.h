@@ -245,10 +245,10 @@ int w2d_flush_l2(W2dCtx* ctx);
  * pointer, block-major [nblocks][neq][20][20], i fastest) whose levels are
  * lev (device pointer, nblocks ints, 1..nlevs); dx, dy are host arrays of
  * nlevs spacings; dt (host) receives the CFL time step.  FP64 only, not for
- * COOLINGDMC.  Nothing is allocated: the per-block partials live in a
- * file-scope device array of W2D_NOALLOC_MAX_BLOCKS doubles that every GPU
- * loading the library keeps until exit; nblocks above that is rejected with
- * W2D_ERR_CAPACITY.  Every call looks up that array's device address
+ * COOLINGDMC.  Nothing is allocated: the running minimum and the result
+ * live in a file-scope device array of W2D_NOALLOC_MAX_BLOCKS doubles that
+ * every GPU loading the library keeps until exit; nblocks above that is
+ * rejected with W2D_ERR_CAPACITY.  Every call looks up that array's device address
  * (cudaGetSymbolAddress, which allocates nothing) in the caller's current
  * device and context, so a host that resets its device or has its context
  * rebuilt by an offload runtime still gets a valid address; the first call
@@ -466,8 +466,10 @@ int w2d_part_halo(const int32_t* innerbounds, int ld, int n, const int32_t* owne
 
 /* ---- Launch shapes and step graphs (no counterpart in the reference) ------
  * The per-leaf kernels (half step, full step, boundaryI, cooling, block
- * statistics) run with one CTA per leaf or on a persistent grid of 2, 4 or
- * 8 CTAs per SM walking the leaves strided or in contiguous chunks.
+ * statistics) run with one CTA per leaf or on a persistent grid of 2 to 8
+ * CTAs per SM walking the leaves strided or in contiguous chunks (grids in
+ * whole waves of the CTAs an SM holds: half and full step 2, 4 and 8, or 2, 3
+ * and 6 where three fit; fill I 2, 6 and 8; cooling 2, 3 and 6).
  * w2d_autotune(ctx, reps) tries every shape for `reps` steps of the live
  * run (results do not depend on the shape) and then keeps the fastest per
  * kernel; w2d_tuning reports, per kernel (half, full, fill I, cooling,
@@ -476,7 +478,10 @@ int w2d_part_halo(const int32_t* innerbounds, int ld, int n, const int32_t* owne
  * makes an ensemble context, or the context of a single run without the
  * jet (w2d_sim_ctx), replay each step's two launch sequences as CUDA
  * graphs (persistent shapes only; leaf count and dt are read on the
- * device, dt reaches the host with the step's synchronization).
+ * device, dt reaches the host with the step's synchronization).  Runs without
+ * admesh and without the jet queue up to 128 steps between two
+ * synchronizations, with the same results; the first failing step's error is
+ * the call's.
  * w2d_set_step_kernel(ctx, 1) lets such a single adiabatic run take each
  * step -- timestep, tstep and the block statistics -- as ONE cooperative
  * persistent kernel whose phases wait on per-block flags instead of kernel
