@@ -476,21 +476,21 @@ void plan_pack(const W2dCtx* c, int2* pf1, int2* pf2, const int* leaves, int nl,
   }
 }
 
-// room in the list of cells left to the exact routine; false: the buffer
-// moved (a captured graph that holds it is stale)
-int ensure_fb(W2dCtx* c, bool* moved)
+// Room in the list of cells left to the exact routine.  A list that has
+// become too short is freed and made anew: the captured steps, which hold its
+// address, go with it.  (Not called while a step is captured.)
+int ensure_fb(W2dCtx* c)
 {
   const int64_t need = (int64_t)c->nleaf * 320;
-  if (moved) *moved = false;
   if (need <= c->fb_cap) return W2D_OK;
   CK(cudaStreamSynchronize(c->st));
+  drop_step_graphs(c);
   if (c->d_fb) cudaFree(c->d_fb);
   c->d_fb = nullptr;
   c->fb_cap = 0;
   const int64_t cap = need + need / 2 + 4096;
   CK(cudaMalloc(&c->d_fb, sizeof(int) * (size_t)cap));
   c->fb_cap = cap;
-  if (moved) *moved = true;
   return W2D_OK;
 }
 
@@ -500,7 +500,7 @@ int ensure_fb(W2dCtx* c, bool* moved)
 int cool_surrogate(W2dCtx* c, const KArgs& a1, const PhysArgs& pa, double dts)
 {
   if (!c->capturing) {
-    int rc0 = ensure_fb(c, nullptr);
+    int rc0 = ensure_fb(c);
     if (rc0) return rc0;
   }
   int rc;
@@ -2061,17 +2061,10 @@ int ctx_step_rest(W2dCtx* c)
   }
   auto body = [&] { return ctx_tstep_rest(c, 0.0, 0.0); };
   if (!graphs_now(c)) return body();
-  if (c->nn_img) {
-    bool moved = false;
-    int rc = ensure_fb(c, &moved);
-    if (rc) return rc;
-    if (moved && c->gx_rest) {
-      cudaGraphExecDestroy(c->gx_rest);
-      c->gx_rest = nullptr;
-    }
-  }
+  int rc;
+  if (c->nn_img && (rc = ensure_fb(c))) return rc;
   if (!c->gx_rest) {
-    int rc = capture(c, &c->gx_rest, &c->nlaunch_graph_rest, body);
+    rc = capture(c, &c->gx_rest, &c->nlaunch_graph_rest, body);
     if (rc) return rc;
   }
   CK(cudaGraphLaunch(c->gx_rest, c->st));
@@ -2107,11 +2100,7 @@ static int queue_steps(W2dCtx* c, int n)
       if ((rc = body())) return rc;
     return W2D_OK;
   }
-  if (c->nn_img) {
-    bool moved = false;
-    if ((rc = ensure_fb(c, &moved))) return rc;
-    if (moved) drop_step_graphs(c);
-  }
+  if (c->nn_img && (rc = ensure_fb(c))) return rc;
   if (!c->gx_whole && (rc = capture(c, &c->gx_whole, &c->nlaunch_graph_whole, body))) return rc;
   for (int k = 0; k < n; ++k) {
     CK(cudaGraphLaunch(c->gx_whole, c->st));
