@@ -93,3 +93,19 @@ def test_fallback_list_moves_between_queued_runs(single_steps, profiled, nets):
         for _ in range(4 if single_steps else 1):
             s.run(1 if single_steps else 4)
     _same("single", a, b)
+
+
+@pytest.mark.parametrize("kind", ["single", "ensemble"])
+def test_tolerance_between_queued_runs(kind, nets):
+    a, b = _pair(kind)
+    for s in (a, b):
+        s.ctx.set_surrogate(nets[0])
+        s.ctx.set_surrogate_tol(0.05)
+        s.run(4)
+        before = s.ctx.surrogate_counts()
+        s.ctx.set_surrogate_tol(1e-6)
+        s.run(4)
+        after = s.ctx.surrogate_counts()
+    _same(kind, a, b)
+    # (the two tolerances serve different shares, so an old one would show)
+    assert before[0] > after[0] - before[0]

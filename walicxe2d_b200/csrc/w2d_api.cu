@@ -147,13 +147,21 @@ int launch_tk(W2dCtx* c, int tk, const char* name, F fn)
   return rc;
 }
 
-// the captured sequences of the separate kernels' steps
+// the captured sequences of the separate kernels' steps that hold what
+// cooling is launched with (the network, its tolerance, the fallback list)
+void drop_cooling_graphs(W2dCtx* c)
+{
+  if (c->gx_rest) cudaGraphExecDestroy(c->gx_rest);
+  if (c->gx_whole) cudaGraphExecDestroy(c->gx_whole);
+  c->gx_rest = c->gx_whole = nullptr;
+}
+
+// all of them
 void drop_step_graphs(W2dCtx* c)
 {
   if (c->gx_first) cudaGraphExecDestroy(c->gx_first);
-  if (c->gx_rest) cudaGraphExecDestroy(c->gx_rest);
-  if (c->gx_whole) cudaGraphExecDestroy(c->gx_whole);
-  c->gx_first = c->gx_rest = c->gx_whole = nullptr;
+  c->gx_first = nullptr;
+  drop_cooling_graphs(c);
 }
 
 // After a synchronization: the tuned kernels' times of the last step go to
@@ -484,7 +492,7 @@ int ensure_fb(W2dCtx* c)
   const int64_t need = (int64_t)c->nleaf * 320;
   if (need <= c->fb_cap) return W2D_OK;
   CK(cudaStreamSynchronize(c->st));
-  drop_step_graphs(c);
+  drop_cooling_graphs(c);
   if (c->d_fb) cudaFree(c->d_fb);
   c->d_fb = nullptr;
   c->fb_cap = 0;
@@ -1885,10 +1893,7 @@ int w2d_set_surrogate_tol(W2dCtx* c, double tol)
 {
   if (!c || !(tol > 0.0) || tol > 0.1) return W2D_ERR_ARG;
   c->nn_tol = (float)tol;
-  if (c->gx_rest) {   // the tolerance is an argument of a captured launch
-    cudaGraphExecDestroy(c->gx_rest);
-    c->gx_rest = nullptr;
-  }
+  drop_cooling_graphs(c);   // the tolerance is an argument of a captured launch
   return W2D_OK;
 }
 
