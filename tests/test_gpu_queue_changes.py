@@ -109,3 +109,19 @@ def test_tolerance_between_queued_runs(kind, nets):
     _same(kind, a, b)
     # (the two tolerances serve different shares, so an old one would show)
     assert before[0] > after[0] - before[0]
+
+
+@pytest.mark.parametrize("single_steps", [False, True])
+@pytest.mark.parametrize("kind", ["single", "ensemble"])
+def test_surrogate_attached_replaced_and_taken_off(kind, single_steps, nets):
+    a, b = _pair(kind)
+    for s in (a, b):
+        for nn in (None, nets[0], nets[1], None):
+            s.ctx.set_surrogate(nn)
+            if single_steps:
+                s.run(1)
+                s.run(1)
+            else:
+                s.run(2)
+    _same(kind, a, b)
+    assert a.ctx.surrogate_counts()[0] > 0

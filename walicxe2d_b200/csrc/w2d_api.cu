@@ -1879,13 +1879,10 @@ extern "C" {
 int w2d_set_surrogate(W2dCtx* c, W2dNN* nn)
 {
   if (!c) return W2D_ERR_ARG;
-  if (!nn) {
-    c->nn_img = nullptr;
-    return W2D_OK;
-  }
-  if (c->p.precision != 32 || c->p.cooling == W2D_ADIABATIC || w2d_nn_kind(nn) != c->p.cooling)
+  if (nn && (c->p.precision != 32 || c->p.cooling == W2D_ADIABATIC || w2d_nn_kind(nn) != c->p.cooling))
     return set_error(c, W2D_ERR_ARG, 0, 0, 0, "the surrogate serves the cooling routine it was trained on, FP32 path");
-  c->nn_img = nn_image_of(nn);
+  c->nn_img = nn ? nn_image_of(nn) : nullptr;
+  drop_cooling_graphs(c);   // which kernels cool, and the network's address
   return W2D_OK;
 }
 
