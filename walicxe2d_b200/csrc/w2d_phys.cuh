@@ -256,15 +256,17 @@ __device__ __forceinline__ bool riemann(const Phys<R>& ph, R* pl, const R* pr, R
 }
 
 // s max(0, min(|a|, s b)) with s = sign(a) (minmod).  In FP64 the signs move
-// as bits instead of through two multiplications, and the zero comes from
-// the sign of the minimum instead of a comparison (a minimum between -2^-1042
-// and 0 stays: no cell value feels it).
+// as bits instead of through two multiplications.  The minimum is negative
+// exactly where s b is: that comparison needs no wait for the minimum, and a
+// NaN b, for which it fails, stays a NaN (full step of 8,835 blocks: 191.1 us,
+// 193.1 from the minimum's own 64-bit pattern; 190.3 from the minimum's sign
+// bit alone, which took NaNs of one sign for negative numbers).
 __device__ __forceinline__ double minmod(double a, double b)
 {
   const unsigned s = (unsigned)__double2hiint(a) & 0x80000000u;
   const double sb = __hiloint2double(__double2hiint(b) ^ (int)s, __double2loint(b));
   const double m = fminr(fabs(a), sb);
-  const bool neg = (unsigned)__double2hiint(m) > 0x80000000u;
+  const bool neg = sb < 0.;
   return __hiloint2double(neg ? (int)s : __double2hiint(m) ^ (int)s, neg ? 0 : __double2loint(m));
 }
 __device__ __forceinline__ float minmod(float a, float b)
