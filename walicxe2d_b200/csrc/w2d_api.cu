@@ -240,6 +240,7 @@ KArgs kargs(W2dCtx* c, const int2* fd)
   } else if (c->dt_on_device && !a.jet) {  // dt from the reduction's device copy (ctx_set_dt_on_device)
     a.dt_dev = c->d_dt;
   }
+  a.nleaf_queued = c->queueing ? c->d_nleaf : nullptr;
   return a;
 }
 
@@ -2132,7 +2133,9 @@ int ctx_queue_run(W2dCtx* c, int n, int* done, const double** dts)
   memset(c->h_queue, 0, sizeof(int) * (size_t)(2 + runs));
   c->h_queue[1] = 1;
   CK(cudaMemcpyAsync(c->d_queue, c->h_queue, sizeof(int) * (size_t)(2 + runs), cudaMemcpyHostToDevice, c->st));
+  c->queueing = true;
   rc = queue_steps(c, n);
+  c->queueing = false;
   if (!rc) {
     CK(cudaMemcpyAsync(c->h_queue, c->d_queue, sizeof(int) * (size_t)(2 + runs), cudaMemcpyDeviceToHost, c->st));
     rc = sync_and_check(c);

@@ -252,6 +252,7 @@ __global__ void __launch_bounds__(W2D_COOL_THREADS, 3) k_cool(KArgs a, PhysArgs 
   const size_t bs = (size_t)NEQ * W2D_CELLS;
   bar_init_once(bar);
   pdl_begin();
+  if (queue_ended<P>(a)) return;
   uint32_t par = 0;
   const double dt_arg = dt_s;
   for (LeafRange lr = leaf_range<P>(a); lr.li < lr.end; lr.li += lr.step, par ^= 1u) {

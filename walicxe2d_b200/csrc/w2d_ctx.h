@@ -84,6 +84,7 @@ struct W2dCtx {
   double* h_hist = nullptr;     // pinned [hist_cap][runs]
   int* h_queue = nullptr;       // pinned [2 + runs]
   int hist_cap = 0;
+  bool queueing = false;        // the launches under way are queued steps
   cudaGraphExec_t gx_whole = nullptr;
   int64_t nlaunch_graph_whole = 0;
   // the fused step kernel (w2d_step.cuh), allocated by its first use: per
