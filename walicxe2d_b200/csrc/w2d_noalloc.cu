@@ -70,8 +70,12 @@ __device__ __forceinline__ Bounds cell_bounds(double d0, double d1, double d2, d
   const float ke = 0.5f * (fabsf(mx) * u + fabsf(my) * v), er = 2e-6f * (fabsf(E) + ke);
   const float icv = 1.f / (float)ph.cv, g = (float)ph.gamma * inv;
   float plo = fmaxf((E - ke - er) * icv, 0.f), phi = fmaxf((E - ke + er) * icv, 1.1e-15f);
-  // coolingh: the pressure of T >= 1 (uprim)
-  if (H) phi = fmaxf(phi, 1.00001f * fmaxf(2.f * r - (float)d4, 1e-15f) / (float)ph.tempsc);
+  // coolingh: the pressure of T >= 1 (uprim).  Its density 2 rho - u5 can cancel:
+  // three roundings of 2^-24 of the terms, not of the difference
+  if (H) {
+    const float n = (float)d4, dent = 2.f * r - n + 2.5e-7f * (2.f * r + fabsf(n));
+    phi = fmaxf(phi, 1.00001f * fmaxf(dent, 1e-15f) / (float)ph.tempsc);
+  }
   const float clo = sqrt_near(g * plo) * (1.f - 4e-6f), chi = sqrt_near(g * phi) * (1.f + 4e-6f);
   const bool fit = ph.cv > 1e-3 && ph.cv < 1e3 && ph.gamma > 1e-3 && ph.gamma < 1e3 &&
                    (!H || (ph.tempsc > 1e-12 && ph.tempsc < 1e30)) && r <= 1e15f && fabsf(E) <= 1e15f && fabsf(E) >= 1e-12f && fabsf(mx) <= 1e15f && fabsf(my) <= 1e15f &&
