@@ -34,3 +34,17 @@ def test_coolingh_floor_with_neutral_density_near_twice_the_density(neq, eps):
     want = _exact(p, u, lev, DX)
     for shift in (0, 1):
         assert _call(p, u, lev, DX, shift) == (0, want)
+
+
+@pytest.mark.parametrize("kind", ["plain", "hypersonic", "uniform", "ties", "extreme"])
+@pytest.mark.parametrize("cooling", [ADIABATIC, COOLINGH])
+@pytest.mark.parametrize("neq", [4, 5, 6])
+def test_noalloc_is_the_fp64_minimum_on_many_blocks(neq, cooling, kind):
+    n = _blocks()
+    rng = np.random.default_rng([neq, cooling, len(kind)])
+    p = base_params(neq=neq, npas=neq - 4, nlevs=4, cooling=cooling)
+    u = _state(kind, n, neq, rng)
+    lev = rng.integers(1, 5, n).astype(np.int32)
+    want = _exact(p, u, lev, DX)
+    for shift in (0, 1):
+        assert _call(p, u, lev, DX, shift) == (0, want)
