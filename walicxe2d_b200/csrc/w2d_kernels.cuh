@@ -868,6 +868,7 @@ __device__ __forceinline__ bool full_leaf(const KArgs& a, const PhysArgs& pa, do
   // 219 us, barrier stalls 3.7 per issue; so, with the leaf's scalars formed
   // once and its statistics finished behind the last barrier: 198 us, 1.7.)
   R* __restrict__ pb = (pa.cooling == COOL_DMC) ? (R*)a.prim + (size_t)b * bs : nullptr;
+  bool got;
   if (tid < 128) {
     const int gf = tid / 32, gg = (tid / 16) % 2;
     int i, j;
@@ -877,22 +878,26 @@ __device__ __forceinline__ bool full_leaf(const KArgs& a, const PhysArgs& pa, do
     bool w = false;
 #pragma unroll
     for (int k = 0; k < NEQ; ++k) w = ghost_value<R>(upool, bs, a, b, d, gf, gg, 1 + tid % 16, k, uu[k]);
-    if (!wait_tiles_p<U>(bar, a.err, b, par)) return false;
-    if (!w) {   // a face no entry writes keeps what it has
+    got = wait_tiles_p(bar, a.err, b, par);
+    if (!U && !got) return false;
+    if (got) {
+      if (!w) {   // a face no entry writes keeps what it has
 #pragma unroll
-      for (int k = 0; k < NEQ; ++k) uu[k] = st[k][j + 1][i + 1];
-    }
-    uprim<NEQ>(ph, q, uu, T);
+        for (int k = 0; k < NEQ; ++k) uu[k] = st[k][j + 1][i + 1];
+      }
+      uprim<NEQ>(ph, q, uu, T);
 #pragma unroll
-    for (int k = 0; k < NEQ; ++k) {
-      u[k * W2D_CELLS + cidx(i, j)] = uu[k];
-      st[k][j + 1][i + 1] = q[k];
-      if (pb != nullptr && gg == 1) pb[k * W2D_CELLS + cidx(i, j)] = q[k];
+      for (int k = 0; k < NEQ; ++k) {
+        u[k * W2D_CELLS + cidx(i, j)] = uu[k];
+        st[k][j + 1][i + 1] = q[k];
+        if (pb != nullptr && gg == 1) pb[k * W2D_CELLS + cidx(i, j)] = q[k];
+      }
     }
   } else {
-    if (!wait_tiles_p<U>(bar, a.err, b, par)) return false;
+    got = wait_tiles_p(bar, a.err, b, par);
+    if (!U && !got) return false;
     const bool jetted = a.jet && a.jetblk[li];
-    for (int c = tid - 128; c < 256; c += W2D_THREADS - 128) {
+    for (int c = tid - 128; c < 256 && got; c += W2D_THREADS - 128) {
       const int i = 1 + c % 16, j = 1 + c / 16;
       R uu[NEQ], q[NEQ], T;
 #pragma unroll
@@ -906,7 +911,9 @@ __device__ __forceinline__ bool full_leaf(const KArgs& a, const PhysArgs& pa, do
       for (int k = 0; k < NEQ; ++k) st[k][j + 1][i + 1] = q[k];
     }
   }
-  __syncthreads();
+  // (one barrier for both sides, which with U also agrees on the outcome)
+  if (!U) __syncthreads();
+  else if (__syncthreads_or(!got)) return false;
 
   // limited fluxes, src/hllcfluxes.f90:50-88: interface tid of x, then of y,
   // through one loop body as in the half step, except with van Leer's limiter,
