@@ -147,21 +147,20 @@ int launch_tk(W2dCtx* c, int tk, const char* name, F fn)
   return rc;
 }
 
-// the captured sequences of the separate kernels' steps that hold what
+// the captured sequence of the separate kernels' steps that holds what
 // cooling is launched with (the network, its tolerance, the fallback list)
-void drop_cooling_graphs(W2dCtx* c)
+void drop_cooling_graph(W2dCtx* c)
 {
   if (c->gx_rest) cudaGraphExecDestroy(c->gx_rest);
-  if (c->gx_whole) cudaGraphExecDestroy(c->gx_whole);
-  c->gx_rest = c->gx_whole = nullptr;
+  c->gx_rest = nullptr;
 }
 
-// all of them
+// both of them
 void drop_step_graphs(W2dCtx* c)
 {
   if (c->gx_first) cudaGraphExecDestroy(c->gx_first);
   c->gx_first = nullptr;
-  drop_cooling_graphs(c);
+  drop_cooling_graph(c);
 }
 
 // After a synchronization: the tuned kernels' times of the last step go to
@@ -493,7 +492,7 @@ int ensure_fb(W2dCtx* c)
   const int64_t need = (int64_t)c->nleaf * 320;
   if (need <= c->fb_cap) return W2D_OK;
   CK(cudaStreamSynchronize(c->st));
-  drop_cooling_graphs(c);
+  drop_cooling_graph(c);
   if (c->d_fb) cudaFree(c->d_fb);
   c->d_fb = nullptr;
   c->fb_cap = 0;
@@ -557,7 +556,8 @@ int half_step(W2dCtx* c, double dt, const double* dt_dev)
 
 static DtPublish dt_publish(W2dCtx* c, double* dt_host)
 {
-  return {dt_host, c->h_err, c->d_err, c->d_queue, c->h_hist, c->hist_cap, std::max(c->nruns, 1), c->d_nleaf};
+  int* steps = c->queueing ? c->d_steps : nullptr;
+  return {dt_host, c->h_err, c->d_err, steps, c->h_steps, c->h_hist, W2D_QUEUE_STEPS, std::max(c->nruns, 1), c->d_nleaf};
 }
 
 // src/timestep.f90:7-61 as one reduction kernel; dt stays in device memory,
@@ -597,7 +597,7 @@ int ctx_dt_launch(W2dCtx* c)
 {
   int rc = dt_reduce(c, dt_publish(c, c->h_small));
   if (rc) return rc;
-  if (!c->capturing) CK(cudaEventRecord(c->ev_dt, c->st));
+  if (!c->capturing && !c->queueing) CK(cudaEventRecord(c->ev_dt, c->st));
   return W2D_OK;
 }
 
@@ -767,7 +767,7 @@ int w2d_create(const W2dParams* p, W2dCtx** out)
   CKC(cudaMalloc(&c->d_cfl, sizeof(double) * slots));
   CKC(cudaMalloc(&c->d_dtcool, sizeof(double) * slots));
   CKC(cudaMalloc(&c->d_grad, sizeof(double) * slots));
-  CKC(cudaMalloc(&c->d_err, sizeof(int) * 4));
+  CKC(cudaMalloc(&c->d_err, sizeof(int) * 5));   // and the queue's count
   CKC(cudaMalloc(&c->d_dt, sizeof(double) * 4));
   CKC(cudaMalloc(&c->d_cooltab, sizeof(double) * 82));
   CKC(cudaMalloc(&c->d_leaves, sizeof(int) * slots));
@@ -786,7 +786,7 @@ int w2d_create(const W2dParams* p, W2dCtx** out)
   cudaDeviceGetAttribute(&c->nsm, cudaDevAttrMultiProcessorCount, c->device);
   CKC(cudaMemsetAsync(c->d_lev, 0, sizeof(int) * slots, c->st));
   CKC(cudaMemsetAsync(c->d_icoord, 0, sizeof(int) * 2 * slots, c->st));
-  CKC(cudaMemsetAsync(c->d_err, 0, sizeof(int) * 4, c->st));
+  CKC(cudaMemsetAsync(c->d_err, 0, sizeof(int) * 5, c->st));
   CKC(cudaMemsetAsync(c->d_cooltab, 0, sizeof(double) * 82, c->st));
   {
     std::vector<double> big(slots, 1e30);
@@ -805,8 +805,11 @@ int w2d_create(const W2dParams* p, W2dCtx** out)
     const unsigned long long w2[2] = {bits, bits};
     CKC(cudaMemcpy(c->d_dtwork, w2, sizeof(w2), cudaMemcpyHostToDevice));
   }
-  CKC(cudaMallocHost(&c->h_small, sizeof(double) * 8));
-  CKC(cudaMallocHost(&c->h_err, sizeof(int) * 4));
+  CKC(cudaMallocHost(&c->h_small, sizeof(double) * (8 + W2D_QUEUE_STEPS)));
+  CKC(cudaMallocHost(&c->h_err, sizeof(int) * 5));
+  c->d_steps = c->d_err + 4;
+  c->h_steps = c->h_err + 4;
+  c->h_hist = c->h_small + 8;
   CKC(cudaMallocHost(&c->h_grad, sizeof(double) * slots));
   CKC(cudaMallocHost(&c->lev, sizeof(int) * slots));
   CKC(cudaMallocHost(&c->icoord, sizeof(int) * 2 * slots));
@@ -828,7 +831,7 @@ int w2d_create(const W2dParams* p, W2dCtx** out)
   CKC(cudaMalloc(&c->d_jetblk, sizeof(int) * slots));
   CKC(cudaEventCreateWithFlags(&c->ev_plan[0], cudaEventDisableTiming));
   CKC(cudaEventCreateWithFlags(&c->ev_plan[1], cudaEventDisableTiming));
-  memset(c->h_err, 0, sizeof(int) * 4);
+  memset(c->h_err, 0, sizeof(int) * 5);
   memset(c->lev, 0, sizeof(int) * slots);
   memset(c->icoord, 0, sizeof(int) * 2 * slots);
 #undef CKC
@@ -861,12 +864,10 @@ int w2d_destroy(W2dCtx* c)
   void* dev2[] = {c->d_run_of, c->d_runs, c->d_dt_run, c->d_loff, c->d_gradleaf, c->d_fb, c->d_fb_count,
                   c->d_nn_counts, c->d_nleaf, c->d_links, c->d_sons, c->d_mflags, c->d_mlists, c->d_rows7,
                   c->d_posof, c->d_bent, c->d_bspan, c->d_blocal, c->d_bcta, c->d_wpos,
-                  c->d_step_flags, c->d_step_sync, c->d_step_part, c->d_queue};
+                  c->d_step_flags, c->d_step_sync, c->d_step_part};
   for (void* d : dev2)
     if (d) cudaFree(d);
   if (c->h_dt_run) cudaFreeHost(c->h_dt_run);
-  if (c->h_queue) cudaFreeHost(c->h_queue);
-  if (c->h_hist) cudaFreeHost(c->h_hist);
   if (c->h_mlists) cudaFreeHost(c->h_mlists);
   if (c->h_rows7) cudaFreeHost(c->h_rows7);
   if (c->h_loff) cudaFreeHost(c->h_loff);
@@ -1763,13 +1764,15 @@ int ctx_set_runs(W2dCtx* c, int nruns, const int* base, const int* cap, const do
   }
   CK(cudaMalloc(&c->d_run_of, sizeof(int) * slots));
   CK(cudaMalloc(&c->d_runs, sizeof(RunGeo) * (size_t)nruns));
-  CK(cudaMalloc(&c->d_dt_run, sizeof(double) * (size_t)nruns));
+  CK(cudaMalloc(&c->d_dt_run, (sizeof(double) + sizeof(int)) * (size_t)nruns));   // and the queue's counts
   CK(cudaMalloc(&c->d_loff, sizeof(int) * (size_t)(nruns + 1)));
-  CK(cudaMallocHost(&c->h_dt_run, sizeof(double) * (size_t)nruns));
+  CK(cudaMallocHost(&c->h_dt_run, sizeof(double) * (size_t)nruns * (1 + W2D_QUEUE_STEPS)));
   CK(cudaMallocHost(&c->h_loff, sizeof(int) * (size_t)(nruns + 1)));
   CK(cudaMemcpy(c->d_run_of, run_of.data(), sizeof(int) * slots, cudaMemcpyHostToDevice));
   CK(cudaMemcpy(c->d_runs, geo.data(), sizeof(RunGeo) * (size_t)nruns, cudaMemcpyHostToDevice));
-  CK(cudaMemset(c->d_dt_run, 0, sizeof(double) * (size_t)nruns));
+  CK(cudaMemset(c->d_dt_run, 0, (sizeof(double) + sizeof(int)) * (size_t)nruns));
+  c->d_steps = reinterpret_cast<int*>(c->d_dt_run + nruns);
+  c->h_hist = c->h_dt_run + nruns;
   c->nruns = nruns;
   c->nbmax = c->cap;
   return W2D_OK;
@@ -1883,7 +1886,7 @@ int w2d_set_surrogate(W2dCtx* c, W2dNN* nn)
   if (nn && (c->p.precision != 32 || c->p.cooling == W2D_ADIABATIC || w2d_nn_kind(nn) != c->p.cooling))
     return set_error(c, W2D_ERR_ARG, 0, 0, 0, "the surrogate serves the cooling routine it was trained on, FP32 path");
   c->nn_img = nn ? nn_image_of(nn) : nullptr;
-  drop_cooling_graphs(c);   // which kernels cool, and the network's address
+  drop_cooling_graph(c);   // which kernels cool, and the network's address
   return W2D_OK;
 }
 
@@ -1891,7 +1894,7 @@ int w2d_set_surrogate_tol(W2dCtx* c, double tol)
 {
   if (!c || !(tol > 0.0) || tol > 0.1) return W2D_ERR_ARG;
   c->nn_tol = (float)tol;
-  drop_cooling_graphs(c);   // the tolerance is an argument of a captured launch
+  drop_cooling_graph(c);   // the tolerance is an argument of a captured launch
   return W2D_OK;
 }
 
@@ -2076,40 +2079,19 @@ int ctx_step_rest(W2dCtx* c)
 }
 
 // Steps queued without a wait between them: runs whose mesh stays (no
-// admesh) and whose dt stays on the device.  Each step is then one graph of
-// the two sequences above (or their launches); the host waits once per batch
-// and takes the steps' dt from the history the reduction kept.
-constexpr int kQueueSteps = 128;
-
+// admesh) and whose dt stays on the device.  The host waits once per batch
+// and takes the steps' dt from the history the reduction kept.  Their kernels
+// are launched one by one, with step graphs too: the launches run ahead of the
+// GPU, and chained by programmatic dependence they follow each other closer
+// than replays of a captured step (20 steps of 4x4 blocks 567 us captured, 532
+// so; of an FP32 ensemble of 4 runs 1,865 and 1,842).
 int ctx_queue_max(W2dCtx* c)
 {
   const bool dev_dt = c->nruns > 0 || ctx_device_dt(c);
   if (!dev_dt || c->tune_left > 0 || c->prof || step_fused_ok(c) || !c->have_topology || !c->have_bounds ||
       c->leaves_dirty)
     return 0;
-  return kQueueSteps;
-}
-
-static int queue_steps(W2dCtx* c, int n)
-{
-  int rc;
-  auto body = [&] {
-    int r = c->nruns > 0 ? ctx_ens_dt_launch(c) : ctx_dt_launch(c);
-    if (!r) r = ctx_half_step(c);
-    return r ? r : ctx_tstep_rest(c, 0.0, 0.0);
-  };
-  if (!graphs_now(c)) {
-    for (int k = 0; k < n; ++k)
-      if ((rc = body())) return rc;
-    return W2D_OK;
-  }
-  if (c->nn_img && (rc = ensure_fb(c))) return rc;
-  if (!c->gx_whole && (rc = capture(c, &c->gx_whole, &c->nlaunch_graph_whole, body))) return rc;
-  for (int k = 0; k < n; ++k) {
-    CK(cudaGraphLaunch(c->gx_whole, c->st));
-    c->nlaunch += c->nlaunch_graph_whole;
-  }
-  return W2D_OK;
+  return W2D_QUEUE_STEPS;
 }
 
 int ctx_queue_run(W2dCtx* c, int n, int* done, const double** dts)
@@ -2117,31 +2099,21 @@ int ctx_queue_run(W2dCtx* c, int n, int* done, const double** dts)
   *done = 0;
   *dts = c->h_hist;
   const int runs = std::max(c->nruns, 1);
-  int rc;
-  if (!c->d_queue) {
-    // (allocated once; graphs captured before hold a reduction without it)
-    CK(cudaStreamSynchronize(c->st));
-    drop_step_graphs(c);
-    CK(cudaMalloc(&c->d_queue, sizeof(int) * (size_t)(2 + runs)));
-    CK(cudaMemsetAsync(c->d_queue, 0, sizeof(int) * (size_t)(2 + runs), c->st));
-    CK(cudaMallocHost(&c->h_queue, sizeof(int) * (size_t)(2 + runs)));
-    CK(cudaMallocHost(&c->h_hist, sizeof(double) * (size_t)kQueueSteps * runs));
-    c->hist_cap = kQueueSteps;
-    *dts = c->h_hist;
-  }
-  n = std::min(n, c->hist_cap);
-  memset(c->h_queue, 0, sizeof(int) * (size_t)(2 + runs));
-  c->h_queue[1] = 1;
-  CK(cudaMemcpyAsync(c->d_queue, c->h_queue, sizeof(int) * (size_t)(2 + runs), cudaMemcpyHostToDevice, c->st));
+  int rc = W2D_OK;
+  n = std::min(n, W2D_QUEUE_STEPS);
+  *c->h_steps = 0;
+  CK(cudaMemsetAsync(c->d_steps, 0, sizeof(int) * (size_t)runs, c->st));
   c->queueing = true;
-  rc = queue_steps(c, n);
+  for (int k = 0; k < n && !rc; ++k) {
+    rc = c->nruns > 0 ? ctx_ens_dt_launch(c) : ctx_dt_launch(c);
+    if (!rc) rc = ctx_half_step(c);
+    if (!rc) rc = ctx_tstep_rest(c, 0.0, 0.0);
+  }
   c->queueing = false;
   if (!rc) {
-    CK(cudaMemcpyAsync(c->h_queue, c->d_queue, sizeof(int) * (size_t)(2 + runs), cudaMemcpyDeviceToHost, c->st));
     rc = sync_and_check(c);
-    *done = c->h_queue[2];
+    *done = *c->h_steps;
   }
-  CK(cudaMemsetAsync(c->d_queue, 0, 2 * sizeof(int), c->st));
   if (rc) {   // the count the reduction set to 0 behind the failed step
     c->h_nleaf[0] = c->nleaf;
     CK(cudaMemcpyAsync(c->d_nleaf, c->h_nleaf, sizeof(int), cudaMemcpyHostToDevice, c->st));

@@ -10,6 +10,9 @@
 #include "../../include/w2d.h"
 #include "w2d_launch.h"
 
+// steps queued between two waits (ctx_queue_run)
+constexpr int W2D_QUEUE_STEPS = 128;
+
 struct W2dCtx {
   W2dParams p{};
   int cap = 0;            // largest block ID
@@ -78,15 +81,13 @@ struct W2dCtx {
   bool dt_on_device = false;
   cudaGraphExec_t gx_first = nullptr, gx_rest = nullptr;
   int64_t nlaunch_graph_first = 0, nlaunch_graph_rest = 0;
-  // steps queued without a wait (ctx_queue_*): the counters the time-step
-  // reduction keeps, the dt of every queued step, the graph of a whole step
-  int* d_queue = nullptr;       // [2 + runs] (DtPublish)
-  double* h_hist = nullptr;     // pinned [hist_cap][runs]
-  int* h_queue = nullptr;       // pinned [2 + runs]
-  int hist_cap = 0;
+  // steps queued without a wait (ctx_queue_*): the counts the time-step
+  // reduction keeps and the dt of every queued step, parts of allocations that
+  // every context has (the first queue allocates nothing)
+  int* d_steps = nullptr;       // [runs], behind d_err or d_dt_run
+  int* h_steps = nullptr;       // pinned, behind h_err
+  double* h_hist = nullptr;     // pinned [W2D_QUEUE_STEPS][runs], behind h_small or h_dt_run
   bool queueing = false;        // the launches under way are queued steps
-  cudaGraphExec_t gx_whole = nullptr;
-  int64_t nlaunch_graph_whole = 0;
   // the fused step kernel (w2d_step.cuh), allocated by its first use: per
   // slot the epochs of the last half and full step, the epoch and barrier
   // words, the CTAs' CFL minima; its grid (-1: not sized yet, 0: it does

@@ -15,12 +15,14 @@ __device__ __forceinline__ void publish_dt(const DtPublish& p, int r, double dt)
   p.dt_host[r] = dt;
   if (r == 0)
     for (int k = 0; k < 4; ++k) p.err_host[k] = p.err[k];
-  if (!p.queue || !p.queue[1]) return;
+  if (!p.steps) return;
+  const int k = p.steps[r];
   if (p.err[0]) {
     if (r == 0) *p.nleaf = 0;
-  } else if (p.queue[2 + r] < p.hist_cap) {
-    p.hist[(size_t)p.queue[2 + r] * p.nruns + r] = dt;
-    p.queue[2 + r] += 1;
+  } else if (k < p.hist_cap) {
+    p.hist[(size_t)k * p.nruns + r] = dt;
+    p.steps[r] = k + 1;
+    if (r == 0) *p.steps_host = k + 1;
   }
 }
 

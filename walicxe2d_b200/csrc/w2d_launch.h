@@ -61,18 +61,20 @@ const Launchers& launchers32();
 
 // Where the dt reduction leaves dt (per run) and the error word for the host:
 // pinned memory that the kernel stores to (dt_host null: nowhere).
-// Steps queued without a wait (queue[1] != 0): the dt of the k-th goes to
-// hist[k * nruns + run], k counted in queue[2 + run]; once the error word is
-// set no further step is counted and the leaf count *nleaf becomes 0, so that
-// the kernels of the steps behind the failed one do nothing.
+// Steps queued without a wait (steps not null): the dt of the k-th goes to
+// hist[k * nruns + run], k counted in steps[run] and run 0's count stored to
+// *steps_host; once the error word is set no further step is counted and the
+// leaf count *nleaf becomes 0, so that the kernels of the steps behind the
+// failed one do nothing.
 struct DtPublish {
   double* dt_host;
   int* err_host;
   const int* err;
-  int* queue;      // null: no queue
-  double* hist;    // pinned
-  int hist_cap;    // steps that fit
-  int nruns;       // runs of the context (1 for a single run)
+  int* steps;        // null: no queue
+  int* steps_host;   // pinned
+  double* hist;      // pinned
+  int hist_cap;      // steps that fit
+  int nruns;         // runs of the context (1 for a single run)
   int* nleaf;
 };
 
