@@ -109,18 +109,21 @@ constexpr Shape kShapes[] = {{0, 0}, {2, 0}, {4, 0}, {4, 1}, {8, 0}, {8, 1}};
 constexpr int kNShape = (int)(sizeof(kShapes) / sizeof(kShapes[0]));
 
 // CTAs per SM of a shape's persistent grid.  The cooling kernel holds three
-// per SM (64 registers, 320 threads): its grids of 4 and 8 would leave the
-// last wave a third full (FP32 ensemble of 6,641 leaves: 151 us on 4 per SM,
-// 130 on 3; compiled for 2 per SM 137).  Fill I holds three in FP64 with the
-// criteria: two waves of them in place of 4 (3,385 leaves: 21.0 us on 4 per SM,
-// 20.9 on 3, 19.2 on 6; 8,835: 41.5, 39.6, 39.3).
+// per SM (50 to 64 registers, 320 threads, in every type): its grids of 4 and 8
+// would leave the last wave a third full (FP32 ensemble of 6,641 leaves: 151 us
+// on 4 per SM, 130 on 3; compiled for 2 per SM 137).  Fill I holds three in FP64
+// (74 to 80 registers): two waves of them in place of 4 (8,836 leaves with the
+// criteria 47.3 us on 4 per SM, 43.5 on 6; 4,356 without 26.9 and 25.1).  In
+// FP32 it holds four (64 registers) and keeps 4 (1,024 leaves 8.6 us on 4, 10.7
+// on 6; 4,356 leaves 12.8 and 15.4; 8,836 leaves 20.2 and 21.1; of 6 equations,
+// 4,356 leaves 18.1 and 18.9, an ensemble of 6,641 28.4 and 27.2).
 // The half and full steps' grids of 4 and 8 become 3 and 6 where 3 CTAs fit.
 int shape_per_sm(const W2dCtx* c, int sh, int tk)
 {
   const int per = kShapes[sh].per_sm;
   if ((tk == TK_HALF || tk == TK_FULL) && per >= 4) return per / 4 * step_ctas(tk == TK_FULL, c->neq, c->elem);
   if (tk == TK_COOL && per >= 4) return per * 3 / 4;
-  return tk == TK_FILL1 && per == 4 ? 6 : per;
+  return tk == TK_FILL1 && per == 4 && c->elem == 8 ? 6 : per;
 }
 
 void apply_shape(W2dCtx* c, KArgs& a, int tk)
