@@ -753,15 +753,13 @@ __device__ __forceinline__ bool half_leaf(const KArgs& a, const PhysArgs& pa, do
   __syncthreads();
 
   // interface tid of each direction: x between (i,j) and (i+1,j), then y
-  // between (i,j) and (i,j+1) with the velocities swapped (swapy).  Where it
-  // measured faster, one loop body serves both (cells a stride apart, the
-  // velocity planes exchanged): half the code, fewer instruction cache misses,
-  // but index arithmetic at run time (FP64, 8,835 blocks of 4 equations: 102.7
-  // -> 101.8 us; of 6 equations, 2,080 blocks: 49.2 -> 51.6; FP32, 6,641 blocks
-  // of 6: 55.6 -> 57.3).
+  // between (i,j) and (i,j+1) with the velocities swapped (swapy: the velocity
+  // planes exchanged).  Unrolled: one loop body for both, half the code with
+  // index arithmetic at run time, measured slower (FP64, 8,835 blocks of 4
+  // equations 95.5 -> 100.0 us, 2,080 of 6 39.6 -> 40.4; FP32, 6,641 blocks of 6
+  // 56.6 -> 57.7).
   if (tid < 272) {
-    constexpr int kBodies = (sizeof(R) == 8 && NEQ == 4) ? 1 : 2;
-#pragma unroll kBodies
+#pragma unroll
     for (int dir = 0; dir < 2; ++dir) {
       const int i = dir ? 1 + tid % 16 : tid % 17, j = dir ? tid / 16 : 1 + tid / 17;
       const int c = cidx(i, j), n = dir ? c + W2D_W : c + 1;
@@ -915,10 +913,12 @@ __device__ __forceinline__ bool full_leaf(const KArgs& a, const PhysArgs& pa, do
   if (!U) __syncthreads();
   else if (__syncthreads_or(!got)) return false;
 
-  // limited fluxes, src/hllcfluxes.f90:50-88: interface tid of x, then of y,
-  // through one loop body as in the half step, except with van Leer's limiter,
-  // whose divisions leave no room for the index registers (FP64, 8,835 blocks:
-  // 198.4 -> 198.1 us, FP32, 6,641: 97.7 -> 95.1; van Leer, 535: 40.1 -> 41.8)
+  // limited fluxes, src/hllcfluxes.f90:50-88: interface tid of x, then of y.  One
+  // loop body for both (cells a stride apart, the velocity planes exchanged), half
+  // the code and fewer instruction cache misses (FP64, 8,835 blocks 193.3 -> 191.3
+  // us, 2,080 blocks of 6 equations 66.1 -> 64.2; FP32, 6,641 blocks 100.4 ->
+  // 96.0), except with van Leer's limiter, whose divisions leave no room for the
+  // index registers (535 blocks: 40.1 -> 41.8)
   if (tid < 272) {
     constexpr int kBodies = LIMITER == 2 ? 2 : 1;
 #pragma unroll kBodies
