@@ -1452,11 +1452,10 @@ int w2d_admesh_flags(W2dCtx* c, int32_t* refine, int cap_refine, int* nrefine, i
   a.tol = c->p.tol;
   a.tol2 = c->p.tol2;
   unsigned char* set = c->d_mflags + 3 * plane * (size_t)c->mark_set;
-  c->mark_set ^= 1;
   a.leafp = set;
   a.up = set + plane;
   a.down = set + 2 * plane;
-  a.next = c->d_mflags + 3 * plane * (size_t)c->mark_set;
+  a.next = c->d_mflags + 3 * plane * (size_t)(1 - c->mark_set);
   // the counters and the heads of both lists in one wait; longer lists
   // (rare: a pass that remeshes thousands of blocks) in a second one
   const int head = (int)std::min<size_t>(slots, 2048);
@@ -1479,7 +1478,8 @@ int w2d_admesh_flags(W2dCtx* c, int32_t* refine, int cap_refine, int* nrefine, i
     c->gbar_count += n;
     return e;
   });
-  if (rc) return rc;
+  if (rc) return rc;   // (nothing launched: this set stays zero for the next call)
+  c->mark_set ^= 1;
   CK(cudaStreamSynchronize(c->st));
   tune_collect(c);
   // (a launch whose barrier gave up handed nothing over: the error word says so)
