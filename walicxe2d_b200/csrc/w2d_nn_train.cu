@@ -329,8 +329,6 @@ __global__ void __launch_bounds__(256) k_nn_adam_multi(const float* __restrict__
   }
 }
 
-// Forward pass of count samples (features SoA, ld apart) into out [2][count].
-
 }  // namespace
 
 namespace w2d {
