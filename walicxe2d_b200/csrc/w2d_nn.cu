@@ -230,8 +230,8 @@ struct __align__(128) NNTrainSmem {
   uint16_t dz2[128 * NN_H];
   uint16_t w2t[NN_H * NN_H];
   uint16_t w3t[NN_H * NN_NOUT];
-  float gb1[NN_H], gb2[NN_H], gb3[NN_NOUT];
-  float loss;
+  float gb1[4][NN_H], gb2[4][NN_H];   // bias gradients of a warp's 32 samples
+  float g3[4][3];                     // output biases and the loss
   uint64_t bar;
   uint32_t tmem;
   int ok;
@@ -266,13 +266,9 @@ __global__ void __launch_bounds__(128, 1) k_nn_train(const float* __restrict__ f
     reinterpret_cast<uint4*>(s.w2t)[k] = reinterpret_cast<const uint4*>(img->w2t)[k];
   for (int k = tid; k < (int)(sizeof(s.w3t) / 16); k += 128)
     reinterpret_cast<uint4*>(s.w3t)[k] = reinterpret_cast<const uint4*>(img->w3t)[k];
-  for (int k = tid; k < NN_H; k += 128) s.gb1[k] = s.gb2[k] = 0.f;
-  if (tid < NN_NOUT) s.gb3[tid] = 0.f;
+  for (int k = tid; k < 4 * NN_H; k += 128) (&s.gb1[0][0])[k] = (&s.gb2[0][0])[k] = 0.f;
   for (int k = tid; k < 128 * NN_NOUT; k += 128) s.dout[k] = 0;
-  if (tid == 0) {
-    s.loss = 0.f;
-    mbar_init(&s.bar, 1);
-  }
+  if (tid == 0) mbar_init(&s.bar, 1);
   if (warp == 0) tc_alloc(&s.tmem, C_ALLOC);
   tc_fence_before();
   __syncthreads();
@@ -364,7 +360,7 @@ __global__ void __launch_bounds__(128, 1) k_nn_train(const float* __restrict__ f
     for (int k = 0; k < NN_H; ++k) {
       float x = v[k];
       for (int o = 16; o > 0; o >>= 1) x += __shfl_xor_sync(0xffffffffu, x, o);
-      if (lane == 0) atomicAdd(&s.gb2[k], x);
+      if (lane == 0) s.gb2[warp][k] += x;
     }
     nn_sync();
     if (tid == 0) {
@@ -384,7 +380,7 @@ __global__ void __launch_bounds__(128, 1) k_nn_train(const float* __restrict__ f
     for (int k = 0; k < NN_H; ++k) {
       float x = v[k];
       for (int o = 16; o > 0; o >>= 1) x += __shfl_xor_sync(0xffffffffu, x, o);
-      if (lane == 0) atomicAdd(&s.gb1[k], x);
+      if (lane == 0) s.gb1[warp][k] += x;
     }
     nn_sync();
     if (tid == 0) {
@@ -394,16 +390,22 @@ __global__ void __launch_bounds__(128, 1) k_nn_train(const float* __restrict__ f
     if (!(ok = nn_wait(&s.bar, phase, err))) break;
     first_tile = false;
   }
-  // bias of the output layer and the loss: warp sums
+  // bias of the output layer and the loss: warp sums.  The warps' sums are added
+  // in one order, so that training on one tile at a time repeats bit for bit:
+  // warp 0, which issues the MMAs, last, as shared atomics nearly always added
+  // them (where something else ran on the GPU some came in another order, and
+  // ten trainings gave nine sets of weights, 2e-7 apart; in the order 0, 1, 2, 3
+  // the weights lie 7e-5 from those).  A step of one tile: 39 us with the
+  // atomics, 23 so.
   for (int o = 16; o > 0; o >>= 1) {
     gb3a += __shfl_xor_sync(0xffffffffu, gb3a, o);
     gb3b += __shfl_xor_sync(0xffffffffu, gb3b, o);
     lsum += __shfl_xor_sync(0xffffffffu, lsum, o);
   }
   if (lane == 0) {
-    atomicAdd(&s.gb3[0], gb3a);
-    atomicAdd(&s.gb3[1], gb3b);
-    atomicAdd(&s.loss, lsum);
+    s.g3[warp][0] = gb3a;
+    s.g3[warp][1] = gb3b;
+    s.g3[warp][2] = lsum;
   }
   tc_fence_before();
   __syncthreads();
@@ -426,11 +428,13 @@ __global__ void __launch_bounds__(128, 1) k_nn_train(const float* __restrict__ f
         for (int k = 0; k < NN_H; ++k) atomicAdd(&grad[P_W3 + lane * NN_H + k], v[k]);
     }
     for (int k = tid; k < NN_H; k += 128) {
-      atomicAdd(&grad[P_B1 + k], s.gb1[k]);
-      atomicAdd(&grad[P_B2 + k], s.gb2[k]);
+      atomicAdd(&grad[P_B1 + k], ((s.gb1[1][k] + s.gb1[2][k]) + s.gb1[3][k]) + s.gb1[0][k]);
+      atomicAdd(&grad[P_B2 + k], ((s.gb2[1][k] + s.gb2[2][k]) + s.gb2[3][k]) + s.gb2[0][k]);
     }
-    if (tid < NN_OUT) atomicAdd(&grad[P_B3 + tid], s.gb3[tid]);
-    if (tid == 0) atomicAdd(&grad[P_N], s.loss * inv_batch);
+    if (tid < 3) {
+      const float x = ((s.g3[1][tid] + s.g3[2][tid]) + s.g3[3][tid]) + s.g3[0][tid];
+      atomicAdd(&grad[P_B3 + tid], tid < 2 ? x : x * inv_batch);   // (the loss follows the biases)
+    }
   }
   tc_fence_before();
   __syncthreads();
