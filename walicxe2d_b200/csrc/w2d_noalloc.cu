@@ -148,7 +148,9 @@ __global__ void __launch_bounds__(256) k_cfl_few(const double* __restrict__ u, c
 // lane l taking cells 2 (l % 8) and the next of rows l / 8, 4 + l / 8, ... .
 // For a positive x, RN(dx/x) falls with x, so a block's partial needs only the
 // largest |u|+cs and |v|+cs.  FP32 bounds find the few cells that can hold
-// them (all 256 where a block is uniform); those alone are computed in FP64.
+// them; those alone are computed in FP64, and of a lane's cells with the same
+// values, which the bounds cannot rank, one (20,011 uniform blocks 80 -> 55 us a
+// call, of 5 equations with coolingh 128 -> 77: what blocks of any values take).
 // Bound by the blocks' bytes: 205 MB of sectors for 20,011 blocks of 4 equations
 // (every cell in FP64 with its own divisions, one CTA per block, a second kernel
 // for the minimum: 86 us a call; so 60, the kernel 41.5).  VEC: 16-byte loads (u on a 16-byte
@@ -188,6 +190,16 @@ __global__ void __launch_bounds__(256) k_cfl_min(const double* __restrict__ u, c
       if (bad == 0) bad = b + 1;
       continue;
     }
+    // cells with the values of the lane's cell before them, whose speeds they share
+    unsigned rep = 0;
+#pragma unroll
+    for (int c = 1; c < 8; ++c) {
+      long long d = 0;
+#pragma unroll
+      for (int e = 0; e < NL; ++e)
+        d |= __double_as_longlong(x[c >> 1][e][c & 1]) ^ __double_as_longlong(x[(c - 1) >> 1][e][(c - 1) & 1]);
+      rep |= (unsigned)(d == 0) << c;
+    }
     float uhi[8], vhi[8], ulo = 0.f, vlo = 0.f;
 #pragma unroll
     for (int c = 0; c < 8; ++c) {
@@ -204,6 +216,7 @@ __global__ void __launch_bounds__(256) k_cfl_min(const double* __restrict__ u, c
     unsigned cand = 0;
 #pragma unroll
     for (int c = 0; c < 8; ++c) cand |= (unsigned)(!(uhi[c] < ulo) || !(vhi[c] < vlo)) << c;   // (NaN: a candidate)
+    cand &= ~rep;
     double mu = 0., mv = 0.;
     while (__any_sync(0xffffffffu, cand != 0)) {
       if (cand) {
