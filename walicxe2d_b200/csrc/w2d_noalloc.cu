@@ -150,7 +150,7 @@ __global__ void __launch_bounds__(256) k_cfl_few(const double* __restrict__ u, c
 // largest |u|+cs and |v|+cs.  FP32 bounds find the few cells that can hold
 // them; those alone are computed in FP64, and of a lane's cells with the same
 // values, which the bounds cannot rank, one (20,011 uniform blocks 80 -> 55 us a
-// call, of 5 equations with coolingh 128 -> 77: what blocks of any values take).
+// call, of 5 equations with coolingh 128 -> 68: what blocks of any values take).
 // Bound by the blocks' bytes: 205 MB of sectors for 20,011 blocks of 4 equations
 // (every cell in FP64 with its own divisions, one CTA per block, a second kernel
 // for the minimum: 86 us a call; so 60, the kernel 41.5).  VEC: 16-byte loads (u on a 16-byte
@@ -265,7 +265,10 @@ void launch_cfl(const double* u, const int32_t* lev, int nblocks, const W2dParam
     k_cfl_few<NEQ><<<nblocks, 256>>>(u, lev, p->nlevs, sp, ph, p->cfl, p->psc, p->tsc, work, out);
     return;
   }
-  const int grid = std::min((nblocks + 7) / 8, 3 * nsm);   // three CTAs of 80 registers per SM
+  // Three CTAs of 80 registers per SM, with coolingh two of up to 112 (20,011
+  // blocks of 5 equations: on three per SM, one and a half waves, 75 us, so 68;
+  // capped to three of 84 registers 83)
+  const int grid = std::min((nblocks + 7) / 8, (H ? 2 : 3) * nsm);
   if (((uintptr_t)u & 15) == 0)
     k_cfl_min<NEQ, H, true><<<grid, 256>>>(u, lev, nblocks, p->nlevs, sp, ph, p->cfl, p->psc, p->tsc, work, out);
   else
