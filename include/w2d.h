@@ -469,7 +469,7 @@ int w2d_part_halo(const int32_t* innerbounds, int ld, int n, const int32_t* owne
  * statistics) run with one CTA per leaf or on a persistent grid of 2 to 8
  * CTAs per SM walking the leaves strided or in contiguous chunks (grids in
  * whole waves of the CTAs an SM holds: half and full step 2, 4 and 8, or 2, 3
- * and 6 where three fit; fill I 2, 6 and 8; cooling 2, 3 and 6).
+ * and 6 where three fit; fill I 2, 6 and 8, in FP32 2, 4 and 8; cooling 2, 3 and 6).
  * w2d_autotune(ctx, reps) tries every shape for `reps` steps of the live
  * run (results do not depend on the shape) and then keeps the fastest per
  * kernel; w2d_tuning reports, per kernel (half, full, fill I, cooling,
@@ -480,7 +480,7 @@ int w2d_part_halo(const int32_t* innerbounds, int ld, int n, const int32_t* owne
  * graphs (persistent shapes only; leaf count and dt are read on the
  * device, dt reaches the host with the step's synchronization).  Runs without
  * admesh and without the jet queue up to 128 steps between two
- * synchronizations, with the same results; the first failing step's error is
+ * synchronizations, launched one by one, with the same results; the first failing step's error is
  * the call's.
  * w2d_set_step_kernel(ctx, 1) lets such a single adiabatic run take each
  * step -- timestep, tstep and the block statistics -- as ONE cooperative
