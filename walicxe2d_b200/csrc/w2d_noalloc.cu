@@ -151,6 +151,8 @@ __global__ void __launch_bounds__(256) k_cfl_few(const double* __restrict__ u, c
 // them; those alone are computed in FP64, and of a lane's cells with the same
 // values, which the bounds cannot rank, one (20,011 uniform blocks 80 -> 55 us a
 // call, of 5 equations with coolingh 128 -> 68: what blocks of any values take).
+// Where every block is flat to below 1e-6 and its cells yet differ, all are
+// computed (82 us; with coolingh 117, a thread per cell took 96).
 // Bound by the blocks' bytes: 205 MB of sectors for 20,011 blocks of 4 equations
 // (every cell in FP64 with its own divisions, one CTA per block, a second kernel
 // for the minimum: 86 us a call; so 60, the kernel 41.5).  VEC: 16-byte loads (u on a 16-byte
